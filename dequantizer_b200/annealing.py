@@ -272,9 +272,8 @@ class BatchedAnnealer:
                 active &= iters < self.max_iters
             if not active.any():
                 break
-            halves = torch.from_numpy(self._ranges(self.half_bounds, active)).to(dev)
             n2e_new, e2n_new = n2e.clone(), torch.empty_like(e2n)
-            self._sweep_halves(T, n2e, e2n, n2e_new, e2n_new, halves)
+            self._sweep_active(T, n2e, e2n, n2e_new, e2n_new, active)
             n2e, e2n = n2e_new, e2n_new
             iters += active
             # the Vidal gauge and distance: after every sweep (the reference's
@@ -390,20 +389,27 @@ class BatchedAnnealer:
         self.fp32_sweeps.append(stage(active.copy(), self.fp32_handover, self.fp32_max_sweeps, fp32_update).tolist())
         return a.to(torch.complex128), b.to(torch.complex128)
 
-    def _sweep_halves(self, T, n2e, e2n, n2e_new, e2n_new, halves):
-        """One synchronous / flooding sweep on the listed half-edges (n2e_new
-        holds the old messages elsewhere), then the edge pass."""
+    def _sweep_active(self, T, n2e, e2n, n2e_new, e2n_new, active: np.ndarray):
+        """One synchronous / flooding sweep of the active instances (n2e_new
+        holds the old messages elsewhere), with the edge pass of all."""
         L = self.layout
         src_sel, edge_new, _ = self.topo.device_tables(L.device)
         stream = _lib.stream_handle()
-        n = int(halves.numel())
         max_slice, max_chi = L.max_slice(), L.max_chi()
         chi3 = L.uniform_k3_chi()
         if chi3:
-            _lib.call("dqz_bp_node_update_k3", L.gptr, chi3, 64, T.data_ptr(), n2e.data_ptr(), e2n.data_ptr(),
-                      n2e_new.data_ptr(), src_sel.data_ptr(), halves.data_ptr(), n,
-                      error_flag(L.device).data_ptr(), stream)
+            every = bool(active.all())
+            nodes = (self.all_nodes_dev if every else
+                     torch.from_numpy(self._ranges(self.node_bounds, active)).to(L.device))
+            # the launch's own edge pass covers the listed nodes' messages
+            _lib.call("dqz_bp_sweep_k3", L.gptr, chi3, T.data_ptr(), n2e.data_ptr(), e2n.data_ptr(),
+                      n2e_new.data_ptr(), e2n_new.data_ptr() if every else None, src_sel.data_ptr(),
+                      edge_new.data_ptr(), nodes.data_ptr(), nodes.numel(), error_flag(L.device).data_ptr(), stream)
+            if every:
+                return
         else:
+            halves = torch.from_numpy(self._ranges(self.half_bounds, active)).to(L.device)
+            n = int(halves.numel())
             nb = _lib.lib().dqz_bp_node_scratch_bytes(n, max_slice, max_chi)
             scratch = torch.empty(nb, dtype=torch.uint8, device=L.device) if nb else None
             _lib.call("dqz_bp_node_update", L.gptr, T.data_ptr(), n2e.data_ptr(), e2n.data_ptr(),

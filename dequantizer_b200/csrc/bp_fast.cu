@@ -1,6 +1,7 @@
 // Shape-specialised BP node update for degree-3 nodes with all bonds of
-// dimension CHI (8 or 16) and physical dimension 2, in complex128 (FP64) or
-// complex64 (FP32) -- the workload of random 3-regular graphs.
+// dimension CHI (8 or 16) and physical dimension 2, in complex64 (FP32) -- the
+// workload of random 3-regular graphs (the FP64 form is bp_k3.cu) -- and the
+// FP64 Vidal-gauge absorption of the same shapes.
 //
 // Same arithmetic as tensor_ops.py:36-60 (pass_through_node), organised as
 // small GEMMs on shared memory. One CTA owns one half-edge h = (v, e); for each
@@ -16,6 +17,12 @@
 #include "common.cuh"
 
 using namespace dqz;
+
+namespace dqz {
+// bp_k3.cu: the FP64 form
+int bp_k3_halves(const dqz_graph_t *g, int chi, const void *T, const void *n2e_old, const void *e2n_old, void *n2e_new,
+                 const uint8_t *src_sel, const int32_t *halves, int n, int *error_flag, cudaStream_t stream);
+}  // namespace dqz
 
 namespace {
 
@@ -394,10 +401,7 @@ extern "C" int dqz_bp_node_update_k3(const dqz_graph_t *g, int32_t chi, int32_t 
     return DQZ_ERR_ARG;
   if (n_halves == 0) return DQZ_OK;
   if (precision == 64) {
-    if (chi == 16) return launch_k3<16, double2>(g, tensors, n2e_old, e2n_old, n2e_new, src_sel, halves, n_halves,
-                                                 error_flag, stream);
-    if (chi == 8) return launch_k3<8, double2>(g, tensors, n2e_old, e2n_old, n2e_new, src_sel, halves, n_halves,
-                                               error_flag, stream);
+    return bp_k3_halves(g, chi, tensors, n2e_old, e2n_old, n2e_new, src_sel, halves, n_halves, error_flag, stream);
   } else if (precision == 32) {
     if (chi == 16) return launch_k3<16, float2>(g, tensors, n2e_old, e2n_old, n2e_new, src_sel, halves, n_halves,
                                                 error_flag, stream);

@@ -117,6 +117,17 @@ int dqz_bp_node_update_k3(const dqz_graph_t *g, int32_t chi, int32_t precision, 
                           const uint8_t *src_sel, const int32_t *halves, int32_t n_halves,
                           int32_t *error_flag, cudaStream_t stream);
 
+/* The FP64 node update of those shapes for whole nodes (all three outgoing
+ * messages of every listed node, on the FP64 tensor cores) with the edge pass
+ * of the listed nodes' messages in the same launch: e2n_new[twin(h)] =
+ * edge_new[twin(h)] ? n2e_new[h] : n2e_old[h] (tensor_ops.py:36-76). e2n_new
+ * may be NULL (no edge pass; edge_new is then not read). Bit-identical to
+ * dqz_bp_node_update_k3 with precision 64 and dqz_bp_edge_pass. */
+int dqz_bp_sweep_k3(const dqz_graph_t *g, int32_t chi, const void *tensors, const void *n2e_old,
+                    const void *e2n_old, void *n2e_new, void *e2n_new, const uint8_t *src_sel,
+                    const uint8_t *edge_new, const int32_t *nodes, int32_t n_nodes,
+                    int32_t *error_flag, cudaStream_t stream);
+
 /* Mixed-precision node update on tensor cores for the same shapes with
  * chi = 16: BF16 products, FP32 accumulation, complex64 messages. One CTA per
  * node (all three outgoing messages); `nodes` lists the nodes to update.
