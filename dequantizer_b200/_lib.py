@@ -86,7 +86,7 @@ _SIGNATURES = {
     "dqz_bp_sweep_sliced": (ctypes.c_int, [_G, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P,
                                            _P]),
     "dqz_bp_node_update_k3": (ctypes.c_int, [_G, _I, _I, _P, _P, _P, _P, _P, _P, _I, _P, _P]),
-    "dqz_bp_sweep_k3": (ctypes.c_int, [_G, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P]),
+    "dqz_bp_sweep_k3": (ctypes.c_int, [_G, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _P, _P, _P]),
     "dqz_bp_edge_pass_c64": (ctypes.c_int, [_G, _P, _P, _P, _P, _P]),
     "dqz_bp_node_update_k3_tc": (ctypes.c_int, [_G, _P, _P, _P, _P, _P, _P, _I, _P, _P]),
     "dqz_bp_node_update_k3_umma": (ctypes.c_int, [_G, _P, _P, _P, _P, _P, _P, _I, _P, _P]),
@@ -99,6 +99,7 @@ _SIGNATURES = {
     "dqz_message_changes_c64": (ctypes.c_int, [_G, _P, _P, _P, _P]),
     "dqz_segment_distance": (ctypes.c_int, [_P, _P, _P, _I, _P, _P, _P]),
     "dqz_bp_node_vjp": (ctypes.c_int, [_G, _P, _P, _P, _P, _P, _P, _I, _I, _I, _P, _P]),
+    "dqz_bp_vjp_k3": (ctypes.c_int, [_G, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P]),
     "dqz_qr_batched": (ctypes.c_int, [_P, ctypes.c_int64, _I, _I, _P, _P, _P, _P]),
     "dqz_set_tuning": (ctypes.c_int, [_I, _I]),
     "dqz_sv_set_basis": (ctypes.c_int, [_P, _I, ctypes.c_int64, _P]),

@@ -30,7 +30,7 @@ import torch
 from . import _lib
 from .graph import Node, TensorGraph
 from .layout import GraphLayout
-from .maps import Topology, bp_sweep
+from .maps import Topology, bp_sweep, error_flag
 
 
 class FixedPointProblem:
@@ -55,6 +55,10 @@ class FixedPointProblem:
         self.nodes_dev = torch.arange(L.n_nodes, dtype=torch.int32, device=L.device)
         self._edge_all = torch.ones(max(L.n_halves, 1), dtype=torch.uint8, device=L.device)
         self._scratch = None
+        # shapes of the tensor-core kernels (bp_k3.cu, adjoint_k3.cu): messages
+        # read at the node's own half-edges, and the change of an iteration
+        self._k3 = L.k3_shape()
+        self._own = torch.zeros(max(L.n_halves, 1), dtype=torch.uint8, device=L.device)
         self.last_sweeps = 0
         self.last_adjoint_sweeps = 0
 
@@ -77,9 +81,21 @@ class FixedPointProblem:
         """Flooding sweeps from n2e until the largest node->edge message
         change is <= tol; returns (n2e*, e2n* = swap(n2e*), sweeps)."""
         e2n = self.swap(n2e)
+        L = self.layout
+        src_sel, edge_new, _ = self.topo.device_tables(L.device)
+        change = torch.zeros(1, dtype=torch.float64, device=L.device)
         for it in range(1, max_sweeps + 1):
-            n2e_new, e2n_new = self.sweep(T, n2e, e2n)
-            d = float((n2e_new - n2e).abs().max())
+            if self._k3:  # the sweep kernel measures the change
+                n2e_new, e2n_new = torch.empty_like(n2e), torch.empty_like(e2n)
+                change.zero_()
+                _lib.call("dqz_bp_sweep_k3", L.gptr, *self._k3, T.data_ptr(), n2e.data_ptr(), e2n.data_ptr(),
+                          n2e_new.data_ptr(), e2n_new.data_ptr(), src_sel.data_ptr(), edge_new.data_ptr(),
+                          self.nodes_dev.data_ptr(), L.n_nodes, 0, change.data_ptr(),
+                          error_flag(L.device).data_ptr(), _lib.stream_handle())
+                d = float(change)
+            else:
+                n2e_new, e2n_new = self.sweep(T, n2e, e2n)
+                d = float((n2e_new - n2e).abs().max())
             n2e, e2n = n2e_new, e2n_new
             if d <= tol:
                 self.last_sweeps = it
@@ -91,6 +107,10 @@ class FixedPointProblem:
         """Transposed node update: returns the e2n cotangent arena; adds the
         node-tensor cotangent into t_cot when given."""
         L = self.layout
+        if self._k3:
+            out = torch.zeros_like(e2n)
+            self._vjp_k3(T, e2n, n2e_cot, self._raw_messages(T, e2n), out, t_cot=t_cot)
+            return out
         if self._scratch is None:
             nb = _lib.lib().dqz_bp_node_vjp_scratch_bytes(L.n_nodes, L.max_size())
             self._scratch = torch.empty(max(int(nb), 1), dtype=torch.uint8, device=L.device)
@@ -99,6 +119,48 @@ class FixedPointProblem:
                   _lib.ptr(t_cot), self.nodes_dev.data_ptr(), L.n_nodes, L.max_size(), L.max_chi(),
                   self._scratch.data_ptr(), _lib.stream_handle())
         return out
+
+    def _raw_messages(self, T, e2n) -> torch.Tensor:
+        """Unnormalised outgoing messages of every node (tensor-core shapes)."""
+        L = self.layout
+        raw = torch.empty_like(e2n)
+        _lib.call("dqz_bp_sweep_k3", L.gptr, *self._k3, T.data_ptr(), e2n.data_ptr(), e2n.data_ptr(), raw.data_ptr(),
+                  None, self._own.data_ptr(), None, self.nodes_dev.data_ptr(), L.n_nodes, 1, None,
+                  error_flag(L.device).data_ptr(), _lib.stream_handle())
+        return raw
+
+    def _vjp_k3(self, T, e2n, n2e_cot, raw, out, add=None, change=None, t_cot=None) -> None:
+        L = self.layout
+        _lib.call("dqz_bp_vjp_k3", L.gptr, *self._k3, T.data_ptr(), e2n.data_ptr(), n2e_cot.data_ptr(),
+                  raw.data_ptr(), _lib.ptr(out), _lib.ptr(add), _lib.ptr(change), _lib.ptr(t_cot),
+                  self.nodes_dev.data_ptr(), L.n_nodes, error_flag(L.device).data_ptr(), _lib.stream_handle())
+
+    def solve_adjoint(self, T, e2n, g, tol: float, max_sweeps: int, t_cot) -> torch.Tensor:
+        """x = g + J^H x by transposed sweeps from x = g until the largest
+        change is <= tol * max|g|; adds the tensor cotangent of x into t_cot."""
+        scale = float(g.abs().max()) or 1.0
+        change = torch.zeros(1, dtype=torch.float64, device=g.device)
+        raw = self._raw_messages(T, e2n) if self._k3 else None  # the same in every transposed sweep
+        x = g.clone()
+        it = 0
+        for it in range(1, max_sweeps + 1):
+            if self._k3:
+                x_new = torch.empty_like(x)
+                change.zero_()
+                self._vjp_k3(T, e2n, x, raw, x_new, add=g, change=change)
+                d = float(change)
+            else:
+                x_new = g + self.transposed_sweep(T, e2n, x)
+                d = float((x_new - x).abs().max())
+            x = x_new
+            if d <= tol * scale:
+                break
+        self.last_adjoint_sweeps = it
+        if self._k3:
+            self._vjp_k3(T, e2n, x, raw, None, t_cot=t_cot)
+        else:
+            self.node_vjp(T, e2n, x, t_cot)
+        return x
 
     def transposed_sweep(self, T, e2n, x):
         """J^H x for the flooding sweep map n2e_old -> n2e_new (its node
@@ -144,18 +206,8 @@ class BPFixedPoint(torch.autograd.Function):
             g = g + g_n2e
         if g_e2n is not None:
             g = g + P.swap(g_e2n.contiguous())  # e2n* = swap(n2e*)
-        x = g.clone()
-        scale = float(g.abs().max()) or 1.0
-        it = 0
-        for it in range(1, ctx.adj_max + 1):
-            x_new = g + P.transposed_sweep(T, e2n, x)
-            d = float((x_new - x).abs().max())
-            x = x_new
-            if d <= ctx.adj_tol * scale:
-                break
-        P.last_adjoint_sweeps = it
         t_cot = torch.zeros_like(T)
-        P.node_vjp(T, e2n, x, t_cot)
+        P.solve_adjoint(T, e2n, g, ctx.adj_tol, ctx.adj_max, t_cot)
         return t_cot, None, None, None, None, None, None
 
 

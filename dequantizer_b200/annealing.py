@@ -402,9 +402,10 @@ class BatchedAnnealer:
             nodes = (self.all_nodes_dev if every else
                      torch.from_numpy(self._ranges(self.node_bounds, active)).to(L.device))
             # the launch's own edge pass covers the listed nodes' messages
-            _lib.call("dqz_bp_sweep_k3", L.gptr, chi3, T.data_ptr(), n2e.data_ptr(), e2n.data_ptr(),
+            _lib.call("dqz_bp_sweep_k3", L.gptr, chi3, 1, T.data_ptr(), n2e.data_ptr(), e2n.data_ptr(),
                       n2e_new.data_ptr(), e2n_new.data_ptr() if every else None, src_sel.data_ptr(),
-                      edge_new.data_ptr(), nodes.data_ptr(), nodes.numel(), error_flag(L.device).data_ptr(), stream)
+                      edge_new.data_ptr(), nodes.data_ptr(), nodes.numel(), 0, None,
+                      error_flag(L.device).data_ptr(), stream)
             if every:
                 return
         else:

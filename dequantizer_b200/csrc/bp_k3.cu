@@ -34,7 +34,7 @@
 // (SPLIT: a wave of small launches is shorter when the three outputs of a node
 // run on three SMs), runs only the three products of that output, in the same
 // order, so every form gives the same bits.
-#include "dmma.cuh"
+#include "k3.cuh"
 
 using namespace dqz;
 
@@ -42,37 +42,17 @@ namespace {
 
 enum K3Mode { NODES, HALVES, SPLIT };
 
-template <int CHI>
-struct K3Cfg {
-  static constexpr int WARPS = CHI == 16 ? 8 : 4;
-  static constexpr int THREADS = 32 * WARPS;
-  static constexpr int TN = CHI / 8;
-  static constexpr int S2 = CHI * CHI, S3 = CHI * S2;
-  static constexpr int SB = CHI + 1;        // slab strides, odd: see dmma.cuh
-  static constexpr int SA = CHI * SB + 1;
-  static constexpr int SLAB = CHI * SA;
-  static constexpr int MS = CHI + 1;        // message row stride
-  static constexpr size_t SMEM = (3 * (size_t)SLAB + 3 * (size_t)CHI * MS) * sizeof(cd);
-  static constexpr int MIN_BLOCKS = CHI == 16 ? 1 : 5;
-};
-
-// One item's table entries (a node and its three half-edges).
-struct K3Item {
-  int ok, mask;         // supported shape; outputs to compute, bit e
-  long long toff;       // node tensor
-  long long hoff[3];    // messages of the node's half-edges
-  const cd *msg[3];     // incoming messages
-  long long twoff[3];   // messages of the far ends' half-edges, -1 without one
-  int new_edge[3];      // the far end reads this sweep's message (edge pass)
-};
-
-template <int CHI, K3Mode MODE>
+// `raw`: the outputs without the division by the trace (then no edge pass).
+// `change`: the largest |n2e_new - n2e_old| entry, as its bits (non-negative
+// doubles order like integers; a NaN orders above all of them and stays).
+template <int CHI, K3Mode MODE, bool FULL>
 __global__ void __launch_bounds__(K3Cfg<CHI>::THREADS, K3Cfg<CHI>::MIN_BLOCKS)
     bp_k3_dmma(dqz_graph_t g, const cd *__restrict__ T, const cd *n2e_old, const cd *e2n_old, cd *n2e_new, cd *e2n_new,
                const uint8_t *__restrict__ src_sel, const uint8_t *__restrict__ edge_new,
-               const int32_t *__restrict__ items, int n_items, int *error_flag) {
+               const int32_t *__restrict__ items, int n_items, int raw, unsigned long long *change,
+               int *error_flag) {
   typedef K3Cfg<CHI> C;
-  constexpr int TN = C::TN, SB = C::SB, SA = C::SA, MS = C::MS, S2 = C::S2, S3 = C::S3, NT = C::THREADS;
+  constexpr int TN = C::TN, SB = C::SB, SA = C::SA, MS = C::MS, S2 = C::S2, NT = C::THREADS;
   constexpr int PER = CHI / C::WARPS;
   typedef CTile<TN, TN> Tile;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -83,8 +63,8 @@ __global__ void __launch_bounds__(K3Cfg<CHI>::THREADS, K3Cfg<CHI>::MIN_BLOCKS)
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
 
   // next item's table entries, thread q < 3 for half-edge q, one dependent level a call
-  int c_it = -1, c_e = 0, c_v = 0, c_h0 = 0, c_ok = 0, c_he = 0, c_sel = 0, c_tw = 0, c_new = 0, c_chi = 0;
-  long long c_toff = 0, c_hoff = 0, c_twoff = 0;
+  int c_it = -1, c_e = 0, c_v = 0, c_h0 = 0, c_k = 0, c_d = 0, c_he = -1, c_sel = 0, c_tw = -1, c_new = 0, c_chi = 0;
+  long long c_toff = 0, c_hoff = 0, c_twoff = -1;
   auto level0 = [&](int i) {
     c_it = items[MODE == SPLIT ? i / 3 : i];
     c_e = MODE == SPLIT ? i % 3 : 0;
@@ -92,11 +72,14 @@ __global__ void __launch_bounds__(K3Cfg<CHI>::THREADS, K3Cfg<CHI>::MIN_BLOCKS)
   auto level1 = [&]() { c_v = MODE == HALVES ? g.half_node[c_it] : c_it; };
   auto level2 = [&]() {
     c_h0 = g.node_half[c_v];
-    c_ok = g.node_degree[c_v] == 3 && g.node_phys[c_v] == 2;
+    c_k = g.node_degree[c_v];
+    c_d = g.node_phys[c_v];
     c_toff = g.node_off[c_v];
   };
   auto level3 = [&]() {
-    if (!c_ok) return;
+    c_he = c_tw = -1;
+    c_sel = DQZ_SRC_E2N_OLD;
+    if (c_k != 3) return;
     const int h = c_h0 + tid;
     c_he = g.half_edge[h];
     c_sel = src_sel[h];
@@ -104,49 +87,28 @@ __global__ void __launch_bounds__(K3Cfg<CHI>::THREADS, K3Cfg<CHI>::MIN_BLOCKS)
     c_tw = g.half_twin[h];
   };
   auto level4 = [&]() {
-    if (!c_ok) return;
     c_chi = c_he >= 0 ? g.edge_chi[c_he] : 0;
     c_twoff = c_tw >= 0 ? g.half_msg_off[c_tw] : -1;
     c_new = (e2n_new && c_tw >= 0) ? edge_new[c_tw] : 0;
   };
   auto publish = [&](K3Item &m) {
-    if (tid == 0) {
-      m.toff = c_toff;
-      m.mask = MODE == NODES ? 7 : 1 << (MODE == HALVES ? c_it - c_h0 : c_e);
-    }
+    const bool own = c_sel == DQZ_SRC_E2N_OLD;
+    m.q[tid] = c_chi;
     m.hoff[tid] = c_hoff;
     m.twoff[tid] = c_twoff;
     m.new_edge[tid] = c_new;
-    const bool own = c_sel == DQZ_SRC_E2N_OLD;
     m.msg[tid] = (own ? e2n_old : (c_sel == DQZ_SRC_N2E_NEW ? n2e_new : n2e_old)) + (own ? c_hoff : c_twoff);
-    const bool fine = c_ok && c_chi == CHI && (own || c_twoff >= 0);
-    const unsigned all = __ballot_sync(0x7u, fine);
-    if (tid == 0) m.ok = all == 0x7u;
+    const bool shape = c_k == 3 && (FULL ? c_d == 2 && c_chi == CHI : c_chi >= 1 && c_chi <= CHI);
+    const unsigned all = __ballot_sync(0x7u, shape && (own || c_twoff >= 0));
+    if (tid == 0) {
+      m.ok = all == 0x7u;
+      m.toff = c_toff;
+      m.d = c_d;
+      m.mask = MODE == NODES ? 7 : 1 << (MODE == HALVES ? c_it - c_h0 : c_e);
+    }
   };
-  auto load_slab = [&](const K3Item &m, int s, cd *dst) {
-    const cd *src = T + m.toff + s;
-#pragma unroll 4
-    for (int i = tid; i < S3; i += NT) cp_async16(dst + (i / S2) * SA + ((i / CHI) % CHI) * SB + i % CHI, src + 2 * i);
-    cp_async_commit();
-  };
-  constexpr int MPT = (S2 + NT - 1) / NT;  // message entries per thread
-  auto load_msgs = [&](const K3Item &m, cd (&x)[3][MPT]) {
-#pragma unroll
-    for (int q = 0; q < 3; ++q)
-#pragma unroll
-      for (int j = 0; j < MPT; ++j) {
-        const int i = tid + j * NT;
-        if (i < S2) x[q][j] = m.msg[q][i];
-      }
-  };
-  auto store_msgs = [&](const cd (&x)[3][MPT]) {
-#pragma unroll
-    for (int q = 0; q < 3; ++q)
-#pragma unroll
-      for (int j = 0; j < MPT; ++j) {
-        const int i = tid + j * NT;
-        if (i < S2) sM[q * CHI * MS + (i / CHI) * MS + i % CHI] = x[q][j];
-      }
+  auto load_msgs = [&](const K3Item &m, cd (&x)[3][C::MPT]) {
+    k3_load_blocks<CHI, FULL>(m, x, [&](int f, int r, int c) { return m.msg[f][r * (FULL ? CHI : m.q[f]) + c]; });
   };
 
   // the first item: everything at once
@@ -161,10 +123,10 @@ __global__ void __launch_bounds__(K3Cfg<CHI>::THREADS, K3Cfg<CHI>::MIN_BLOCKS)
     }
     __syncthreads();
     if (!meta[buf].ok) return;
-    load_slab(meta[buf], 0, dst);
-    cd x[3][MPT];
+    k3_load_slab<CHI, FULL>(T, meta[buf], 0, dst);
+    cd x[3][C::MPT];
     load_msgs(meta[buf], x);
-    store_msgs(x);
+    k3_store_blocks<CHI>(sM, x);
   };
 
   int cur = 0, p = 0;  // p: slab buffer holding T
@@ -180,20 +142,26 @@ __global__ void __launch_bounds__(K3Cfg<CHI>::THREADS, K3Cfg<CHI>::MIN_BLOCKS)
       continue;
     }
     const int mask = MODE == NODES ? 7 : meta[cur].mask;
+    const int d = FULL ? 2 : meta[cur].d;
     Tile o0, o1, o2;  // out_0 transposed, out_1, out_2: this warp's share
     o0.clear();
     o1.clear();
     o2.clear();
-    cd xn[3][MPT];  // the next item's messages
+    cd xn[3][C::MPT];  // the next item's messages
 #pragma unroll 1
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < d; ++s) {
+      const bool last = s == d - 1;
       const cd *sT = slab + p * C::SLAB;
       cd *sE = slab + ((p + 1) % 3) * C::SLAB;
       cd *sD = slab + ((p + 2) % 3) * C::SLAB;
       const cd *m0 = sM, *m1 = sM + CHI * MS, *m2 = sM + 2 * CHI * MS;
       if (tid < 3 && has_next) {
-        if (s == 0) level0(next);
-        else level3();
+        if (FULL && s == 0) level0(next);
+        if (FULL && s == 1) level3();
+        if (!FULL && last) {
+          level0(next);
+          level1();
+        }
       }
       cp_async_wait<0>();
       __syncthreads();
@@ -209,8 +177,12 @@ __global__ void __launch_bounds__(K3Cfg<CHI>::THREADS, K3Cfg<CHI>::MIN_BLOCKS)
         }
       }
       if (tid < 3 && has_next) {
-        if (s == 0) level1();
-        else level4();
+        if (FULL && s == 0) level1();
+        if (FULL && s == 1) level4();
+        if (!FULL && last) {
+          level2();
+          level3();
+        }
       }
       __syncthreads();
 #pragma unroll 1
@@ -236,15 +208,16 @@ __global__ void __launch_bounds__(K3Cfg<CHI>::THREADS, K3Cfg<CHI>::MIN_BLOCKS)
         }
       }
       if (tid < 3 && has_next) {
-        if (s == 0) level2();
-        else publish(meta[cur ^ 1]);
+        if (FULL && s == 0) level2();
+        if (!FULL && last) level4();
+        if (last) publish(meta[cur ^ 1]);
       }
       __syncthreads();
       // E0's buffer takes the next slab
-      if (s == 0) {
-        load_slab(meta[cur], 1, sE);
+      if (!last) {
+        k3_load_slab<CHI, FULL>(T, meta[cur], s + 1, sE);
       } else if (has_next && meta[cur ^ 1].ok) {
-        load_slab(meta[cur ^ 1], 0, sE);
+        k3_load_slab<CHI, FULL>(T, meta[cur ^ 1], 0, sE);
         load_msgs(meta[cur ^ 1], xn);
       }
       if (mask & 1) {
@@ -267,22 +240,12 @@ __global__ void __launch_bounds__(K3Cfg<CHI>::THREADS, K3Cfg<CHI>::MIN_BLOCKS)
     constexpr int WS = C::WARPS * S2;  // one output's shares
     static_assert(2 * WS <= C::SLAB && WS + 3 * CHI * MS <= C::SLAB, "the shares fit two slabs");
     __syncthreads();
-    {
-      auto part = [&](const Tile &o, cd *dst) {
-        int pos = 0;
-#pragma unroll
-        for (int r = 0; r < TN; ++r)
-#pragma unroll
-          for (int n = 0; n < TN; ++n)
-#pragma unroll
-            for (int i = 0; i < 2; ++i) dst[w * S2 + (pos++) * 32 + lane] = mk(o.re[r][n][i], o.im[r][n][i]);
-      };
-      if (mask & 1) part(o0, r0);
-      if (mask & 2) part(o1, r0 + WS);
-      if (mask & 4) part(o2, r2);
-    }
-    if (has_next && meta[cur ^ 1].ok) store_msgs(xn);
+    if (mask & 1) k3_put_share<CHI>(o0, r0 + w * S2);
+    if (mask & 2) k3_put_share<CHI>(o1, r0 + WS + w * S2);
+    if (mask & 4) k3_put_share<CHI>(o2, r2 + w * S2);
+    if (has_next && meta[cur ^ 1].ok) k3_store_blocks<CHI>(sM, xn);
     __syncthreads();
+    const K3Item &m = meta[cur];
     cd *fin = r2 + WS;  // 3 x CHI x MS: the summed outputs, row-major
     for (int i = tid; i < 3 * S2; i += NT) {
       const int e = i / S2, x = i % S2;
@@ -291,46 +254,66 @@ __global__ void __launch_bounds__(K3Cfg<CHI>::THREADS, K3Cfg<CHI>::MIN_BLOCKS)
       cd sum = src[0];
 #pragma unroll
       for (int k = 1; k < C::WARPS; ++k) sum = cadd(sum, src[k * S2]);
-      const int pos = x >> 5, ln = x & 31;
-      const int row = 8 * (pos / (2 * TN)) + (ln >> 2), col = 8 * ((pos / 2) % TN) + 2 * (ln & 3) + (pos & 1);
+      int row, col;
+      k3_pos<CHI>(x, row, col);
       fin[e * CHI * MS + (e == 0 ? col * MS + row : row * MS + col)] = sum;
     }
     __syncthreads();
     if (tid < 3 && ((mask >> tid) & 1)) {
       cd tr = czero();
-      for (int i = 0; i < CHI; ++i) tr = cadd(tr, fin[tid * CHI * MS + i * MS + i]);
+      for (int i = 0; i < (FULL ? CHI : m.q[tid]); ++i) tr = cadd(tr, fin[tid * CHI * MS + i * MS + i]);
       trace_sh[tid] = tr;
     }
     __syncthreads();
+    double far = 0.0;
     for (int i = tid; i < 3 * S2; i += NT) {
-      const int e = i / S2, x = i % S2;
+      const int e = i / S2, r = (i % S2) / CHI, c = i % CHI;
       if (!((mask >> e) & 1)) continue;
-      const cd o = cdiv(fin[e * CHI * MS + (x / CHI) * MS + x % CHI], trace_sh[e]);
-      const K3Item &m = meta[cur];
+      const int qe = FULL ? CHI : m.q[e];
+      if (!FULL && (r >= qe || c >= qe)) continue;
+      const int x = r * qe + c;
+      const cd y = fin[e * CHI * MS + r * MS + c];
+      const cd o = raw ? y : cdiv(y, trace_sh[e]);
+      if (change) {
+        const double dist = sqrt(cabs2(csub(o, n2e_old[m.hoff[e] + x])));
+        far = dist > far || dist != dist ? dist : far;
+      }
       n2e_new[m.hoff[e] + x] = o;
       // edge pass: the far end's incoming message
       if (e2n_new && m.twoff[e] >= 0) e2n_new[m.twoff[e] + x] = m.new_edge[e] ? o : n2e_old[m.hoff[e] + x];
+    }
+    if (change) {
+      unsigned long long bits = (unsigned long long)__double_as_longlong(far);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long y = __shfl_xor_sync(0xffffffffu, bits, o);
+        bits = y > bits ? y : bits;
+      }
+      if (lane == 0) atomicMax(change, bits);
     }
     cur ^= 1;
   }
 }
 
-int sm_count() {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
+struct K3Args {
+  const dqz_graph_t *g;
+  const void *T, *n2e_old, *e2n_old;
+  void *n2e_new, *e2n_new;
+  const uint8_t *src_sel, *edge_new;
+  int raw;
+  unsigned long long *change;
+  int *error_flag;
+  cudaStream_t stream;
+};
 
-template <int CHI, K3Mode MODE>
-int launch(const dqz_graph_t *g, const void *T, const void *n2e_old, const void *e2n_old, void *n2e_new, void *e2n_new,
-           const uint8_t *src_sel, const uint8_t *edge_new, const int32_t *items, int n, int *error_flag,
-           cudaStream_t stream) {
+template <int CHI, K3Mode MODE, bool FULL>
+int launch(const K3Args &a, const int32_t *items, int n) {
   typedef K3Cfg<CHI> C;
-  DQZ_SMEM_ATTR_ONCE((bp_k3_dmma<CHI, MODE>), C::SMEM);
-  const int slots = sm_count() * C::MIN_BLOCKS;
-  bp_k3_dmma<CHI, MODE><<<n < slots ? n : slots, C::THREADS, C::SMEM, stream>>>(
-      *g, (const cd *)T, (const cd *)n2e_old, (const cd *)e2n_old, (cd *)n2e_new, (cd *)e2n_new, src_sel, edge_new,
-      items, n, error_flag);
+  DQZ_SMEM_ATTR_ONCE((bp_k3_dmma<CHI, MODE, FULL>), C::SMEM);
+  const int slots = k3_sm_count() * C::MIN_BLOCKS;
+  bp_k3_dmma<CHI, MODE, FULL><<<n < slots ? n : slots, C::THREADS, C::SMEM, a.stream>>>(
+      *a.g, (const cd *)a.T, (const cd *)a.n2e_old, (const cd *)a.e2n_old, (cd *)a.n2e_new, (cd *)a.e2n_new, a.src_sel,
+      a.edge_new, items, n, a.raw, a.change, a.error_flag);
   DQZ_CHECK_LAUNCH();
   return DQZ_OK;
 }
@@ -339,16 +322,12 @@ int launch(const dqz_graph_t *g, const void *T, const void *n2e_old, const void 
 // SPLIT where its waves are the shorter (at most a third of a wave of nodes, or
 // two thirds). Measured at bond 16, us: 49 nodes 24.7 split, 43 whole; 98 nodes
 // 44 split, 43 whole; 99 nodes 62 split, 42 whole; 296 nodes 121 split, 80 whole.
-template <int CHI>
-int sweep(const dqz_graph_t *g, const void *T, const void *n2e_old, const void *e2n_old, void *n2e_new, void *e2n_new,
-          const uint8_t *src_sel, const uint8_t *edge_new, const int32_t *nodes, int n, int *error_flag,
-          cudaStream_t stream) {
-  const long long slots = (long long)sm_count() * K3Cfg<CHI>::MIN_BLOCKS;
-  const bool split = 3 * ((3ll * n + slots - 1) / slots) < 7 * ((n + slots - 1) / slots);
-  if (split)
-    return launch<CHI, SPLIT>(g, T, n2e_old, e2n_old, n2e_new, e2n_new, src_sel, edge_new, nodes, 3 * n, error_flag,
-                              stream);
-  return launch<CHI, NODES>(g, T, n2e_old, e2n_old, n2e_new, e2n_new, src_sel, edge_new, nodes, n, error_flag, stream);
+template <int CHI, bool FULL>
+int sweep(const K3Args &a, const int32_t *nodes, int n) {
+  const long long slots = (long long)k3_sm_count() * K3Cfg<CHI>::MIN_BLOCKS;
+  if (3 * ((3ll * n + slots - 1) / slots) < 7 * ((n + slots - 1) / slots))
+    return launch<CHI, SPLIT, FULL>(a, nodes, 3 * n);
+  return launch<CHI, NODES, FULL>(a, nodes, n);
 }
 
 }  // namespace
@@ -357,28 +336,25 @@ namespace dqz {
 
 int bp_k3_halves(const dqz_graph_t *g, int chi, const void *T, const void *n2e_old, const void *e2n_old, void *n2e_new,
                  const uint8_t *src_sel, const int32_t *halves, int n, int *error_flag, cudaStream_t stream) {
-  if (chi == 16)
-    return launch<16, HALVES>(g, T, n2e_old, e2n_old, n2e_new, nullptr, src_sel, nullptr, halves, n, error_flag, stream);
-  if (chi == 8)
-    return launch<8, HALVES>(g, T, n2e_old, e2n_old, n2e_new, nullptr, src_sel, nullptr, halves, n, error_flag, stream);
+  const K3Args a{g, T, n2e_old, e2n_old, n2e_new, nullptr, src_sel, nullptr, 0, nullptr, error_flag, stream};
+  if (chi == 16) return launch<16, HALVES, true>(a, halves, n);
+  if (chi == 8) return launch<8, HALVES, true>(a, halves, n);
   return DQZ_ERR_UNSUPPORTED;
 }
 
 }  // namespace dqz
 
-extern "C" int dqz_bp_sweep_k3(const dqz_graph_t *g, int32_t chi, const void *tensors, const void *n2e_old,
-                               const void *e2n_old, void *n2e_new, void *e2n_new, const uint8_t *src_sel,
-                               const uint8_t *edge_new, const int32_t *nodes, int32_t n_nodes, int32_t *error_flag,
-                               cudaStream_t stream) {
+extern "C" int dqz_bp_sweep_k3(const dqz_graph_t *g, int32_t max_chi, int32_t uniform, const void *tensors,
+                               const void *n2e_old, const void *e2n_old, void *n2e_new, void *e2n_new,
+                               const uint8_t *src_sel, const uint8_t *edge_new, const int32_t *nodes, int32_t n_nodes,
+                               int32_t raw, double *max_change, int32_t *error_flag, cudaStream_t stream) {
   if (!g || !tensors || !n2e_old || !e2n_old || !n2e_new || !src_sel || !nodes || !error_flag || n_nodes < 0)
     return DQZ_ERR_ARG;
-  if (e2n_new && !edge_new) return DQZ_ERR_ARG;
+  if (e2n_new && (!edge_new || raw)) return DQZ_ERR_ARG;
+  if (max_chi <= 0 || max_chi > 16 || (uniform && max_chi != 8 && max_chi != 16)) return DQZ_ERR_UNSUPPORTED;
   if (n_nodes == 0) return DQZ_OK;
-  if (chi == 16)
-    return sweep<16>(g, tensors, n2e_old, e2n_old, n2e_new, e2n_new, src_sel, edge_new, nodes, n_nodes, error_flag,
-                     stream);
-  if (chi == 8)
-    return sweep<8>(g, tensors, n2e_old, e2n_old, n2e_new, e2n_new, src_sel, edge_new, nodes, n_nodes, error_flag,
-                    stream);
-  return DQZ_ERR_UNSUPPORTED;
+  const K3Args a{g, tensors, n2e_old, e2n_old, n2e_new, e2n_new, src_sel, edge_new, raw,
+                 reinterpret_cast<unsigned long long *>(max_change), error_flag, stream};
+  if (uniform) return max_chi == 16 ? sweep<16, true>(a, nodes, n_nodes) : sweep<8, true>(a, nodes, n_nodes);
+  return max_chi > 8 ? sweep<16, false>(a, nodes, n_nodes) : sweep<8, false>(a, nodes, n_nodes);
 }

@@ -113,7 +113,7 @@ class BPEngine:
     def kernel(self) -> str:
         if self.precision == "bf16":
             return "bp_node_k3_umma" if self.bf16_kernel == "tcgen05" else "bp_node_k3_tc"
-        return "bp_node_k3" if self.layout.uniform_k3_chi() else "bp_node_generic"
+        return "bp_node_k3" if self.layout.k3_shape() else "bp_node_generic"
 
     # -------------------------------------------------------------- load
     def _load_pieces(self, arena: torch.Tensor, offsets, pieces: Sequence) -> None:
@@ -252,9 +252,9 @@ class BPEngine:
                           self.e2n.data_ptr(), n2e_new.data_ptr(), src_sel.data_ptr(), ids.data_ptr(), ids.numel(),
                           flag.data_ptr(), stream)
             else:
-                _lib.call("dqz_bp_sweep_k3", L.gptr, chi, self.T.data_ptr(), self.n2e.data_ptr(),
+                _lib.call("dqz_bp_sweep_k3", L.gptr, chi, 1, self.T.data_ptr(), self.n2e.data_ptr(),
                           self.e2n.data_ptr(), n2e_new.data_ptr(), e2n_new.data_ptr(), src_sel.data_ptr(),
-                          edge_new.data_ptr(), ids.data_ptr(), ids.numel(), flag.data_ptr(), stream)
+                          edge_new.data_ptr(), ids.data_ptr(), ids.numel(), 0, None, flag.data_ptr(), stream)
             down.wait_event(cur.record_event())
             with torch.cuda.stream(down):
                 out_n2e[ma:mb].copy_(n2e_new[ma:mb], non_blocking=True)
@@ -287,10 +287,11 @@ class BPEngine:
         self.n2e, self.e2n = n2e_new, e2n_new
 
     def launches_per_sweep(self) -> int:
-        if len(self.topo.levels) > 1 and self.T.dtype == torch.complex128 and not self.layout.uniform_k3_chi():
-            return 1  # every level and the edge pass in one cooperative launch (dqz_bp_sweep_levels)
-        if self.precision == "fp64" and self.layout.uniform_k3_chi():
-            return len(self.topo.levels)  # the edge pass runs in the node update's launch (dqz_bp_sweep_k3)
+        if self.precision == "fp64":
+            if self.layout.uniform_k3_chi() or (self.layout.k3_shape() and len(self.topo.levels) == 1):
+                return len(self.topo.levels)  # the edge pass runs in the node update's launch (dqz_bp_sweep_k3)
+            if len(self.topo.levels) > 1:
+                return 1  # every level and the edge pass in one cooperative launch (dqz_bp_sweep_levels)
         return len(self.topo.levels) + 1
 
     def check(self) -> None:

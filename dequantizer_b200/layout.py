@@ -77,6 +77,7 @@ class GraphLayout:
                 self.half_twin[a] = b
                 self.half_twin[b] = a
         self.edge_chi = np.array(edge_chi, dtype=np.int32)
+        self._shape_kept = (None, None)
         if m and self.edge_chi.max(initial=1) > _lib.MAX_CHI:
             raise NotImplementedError(f"bond dimension above {_lib.MAX_CHI} is not supported on the GPU")
         self.edge_capacity = np.array(edge_capacity if edge_capacity is not None else self.edge_chi, dtype=np.int64)
@@ -108,18 +109,38 @@ class GraphLayout:
     def half_chi(self) -> np.ndarray:
         return self.edge_chi[self.half_edge]
 
+    def _shape(self):
+        """(max bond, max node size, max bond slice, uniform_k3_chi, k3_shape),
+        kept for the bond dimensions they were computed from: a sweep asks for
+        them on every call, and small graphs' sweeps last a few microseconds."""
+        key = self.edge_chi.tobytes()
+        kept, value = self._shape_kept
+        if key != kept:
+            max_chi = int(self.edge_chi.max(initial=1))
+            sizes = self.node_sizes()
+            max_slice = 1
+            if self.n_halves:
+                max_slice = int((sizes[self.half_node] // np.maximum(self.half_chi(), 1)).max())
+            k3 = bool(self.n_nodes and self.n_edges and np.all(self.degree == 3) and not np.any(self.half_edge < 0))
+            uniform = 0
+            if k3 and np.all(self.phys == 2) and max_chi in (8, 16) and np.all(self.edge_chi == max_chi):
+                uniform = max_chi
+            shape = (max_chi, 1 if uniform else 0) if k3 and max_chi <= 16 else None
+            value = (max_chi, int(sizes.max(initial=1)), max_slice, uniform, shape)
+            self._shape_kept = (key, value)
+        return value
+
     def uniform_k3_chi(self) -> int:
         """Bond dimension when every node has degree 3 and physical dimension
-        2 and every edge the same bond dimension in {8, 16} (the shapes the
-        specialised node-update kernel covers); 0 otherwise."""
-        if not self.n_nodes or not self.n_edges:
-            return 0
-        if not (np.all(self.degree == 3) and np.all(self.phys == 2)):
-            return 0
-        chi = int(self.edge_chi[0])
-        if chi not in (8, 16) or not np.all(self.edge_chi == chi) or np.any(self.half_edge < 0):
-            return 0
-        return chi
+        2 and every edge the same bond dimension in {8, 16} (the shapes with
+        compile-time strides); 0 otherwise."""
+        return self._shape()[3]
+
+    def k3_shape(self):
+        """(largest bond, 1 when ``uniform_k3_chi``) when the degree-3
+        tensor-core kernels cover every node (degree 3, bonds up to 16, zero-
+        padded to 8 or 16 when not uniform); None otherwise."""
+        return self._shape()[4]
 
     # ------------------------------------------------------------ offsets
     def _finish(self):
@@ -193,17 +214,14 @@ class GraphLayout:
 
     # --------------------------------------------------------- capacities
     def max_chi(self) -> int:
-        return int(self.edge_chi.max(initial=1))
+        return self._shape()[0]
 
     def max_size(self) -> int:
-        return int(self.node_sizes().max(initial=1))
+        return self._shape()[1]
 
     def max_slice(self) -> int:
         """Largest bond slice (node size / bond dimension) over all half-edges."""
-        sizes = self.node_sizes()
-        if not self.n_halves:
-            return 1
-        return int((sizes[self.half_node] // np.maximum(self.half_chi(), 1)).max())
+        return self._shape()[2]
 
     # ---------------------------------------------------------- packing
     def new_tensor_arena(self) -> torch.Tensor:

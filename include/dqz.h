@@ -117,16 +117,22 @@ int dqz_bp_node_update_k3(const dqz_graph_t *g, int32_t chi, int32_t precision, 
                           const uint8_t *src_sel, const int32_t *halves, int32_t n_halves,
                           int32_t *error_flag, cudaStream_t stream);
 
-/* The FP64 node update of those shapes for whole nodes (all three outgoing
- * messages of every listed node, on the FP64 tensor cores) with the edge pass
- * of the listed nodes' messages in the same launch: e2n_new[twin(h)] =
- * edge_new[twin(h)] ? n2e_new[h] : n2e_old[h] (tensor_ops.py:36-76). e2n_new
- * may be NULL (no edge pass; edge_new is then not read). Bit-identical to
- * dqz_bp_node_update_k3 with precision 64 and dqz_bp_edge_pass. */
-int dqz_bp_sweep_k3(const dqz_graph_t *g, int32_t chi, const void *tensors, const void *n2e_old,
-                    const void *e2n_old, void *n2e_new, void *e2n_new, const uint8_t *src_sel,
-                    const uint8_t *edge_new, const int32_t *nodes, int32_t n_nodes,
-                    int32_t *error_flag, cudaStream_t stream);
+/* FP64 node update of degree-3 nodes with bonds up to 16 for whole nodes (all
+ * three outgoing messages of every listed node, on the FP64 tensor cores), with
+ * the edge pass of the listed nodes' messages in the same launch:
+ * e2n_new[twin(h)] = edge_new[twin(h)] ? n2e_new[h] : n2e_old[h]
+ * (tensor_ops.py:36-76). `uniform`: every listed node has three bonds of
+ * dimension max_chi (8 or 16) and physical dimension 2; bit-identical to
+ * dqz_bp_node_update_k3 with precision 64. Otherwise bonds up to max_chi (<= 16)
+ * and any physical dimension. A node of another shape is skipped and sets
+ * *error_flag to 1. e2n_new may be NULL (no edge pass; edge_new is then not
+ * read). `raw`: outputs without the division by their trace (no edge pass).
+ * max_change, when not NULL, is raised to the largest |n2e_new - n2e_old| entry
+ * of the listed nodes (the caller sets it to 0; NaN when an entry is NaN). */
+int dqz_bp_sweep_k3(const dqz_graph_t *g, int32_t max_chi, int32_t uniform, const void *tensors,
+                    const void *n2e_old, const void *e2n_old, void *n2e_new, void *e2n_new,
+                    const uint8_t *src_sel, const uint8_t *edge_new, const int32_t *nodes, int32_t n_nodes,
+                    int32_t raw, double *max_change, int32_t *error_flag, cudaStream_t stream);
 
 /* Mixed-precision node update on tensor cores for the same shapes with
  * chi = 16: BF16 products, FP32 accumulation, complex64 messages. One CTA per
@@ -266,6 +272,19 @@ int dqz_bp_node_vjp(const dqz_graph_t *g, const void *tensors, const void *e2n, 
                     void *e2n_cot, void *t_cot, const int32_t *nodes, int32_t n_nodes, int32_t max_size,
                     int32_t max_chi, void *scratch, cudaStream_t stream);
 size_t dqz_bp_node_vjp_scratch_bytes(int32_t n_nodes, int32_t max_size);
+
+/* The same adjoint for degree-3 nodes with bonds up to 16 (shapes and `uniform` as
+ * dqz_bp_sweep_k3), on the FP64 tensor cores. `raw` holds the unnormalised
+ * outgoing messages of (tensors, e2n), from dqz_bp_sweep_k3 with raw != 0.
+ * e2n_cot (may be NULL) receives the cotangents of the incoming messages or,
+ * with `add`, the next iterate of x = add + swap(VJP(x)) for x = n2e_cot (out of
+ * place), *max_change being raised to the largest |next - x| entry. The
+ * tensor cotangents are added into t_cot when it is not NULL. A node of another
+ * shape is skipped and, where e2n_cot is given, sets *error_flag to 1. */
+int dqz_bp_vjp_k3(const dqz_graph_t *g, int32_t max_chi, int32_t uniform, const void *tensors,
+                  const void *e2n, const void *n2e_cot, const void *raw, void *e2n_cot, const void *add,
+                  double *max_change, void *t_cot, const int32_t *nodes, int32_t n_nodes,
+                  int32_t *error_flag, cudaStream_t stream);
 
 /* ---- Batched reduced QR (the QR of tensor_ops.py:288, LAPACK conventions) --
  * For each of `batch` row-major m x k complex128 matrices A_b: A_b = Q_b R_b with

@@ -87,9 +87,9 @@ def test_other_shapes_are_flagged_and_skipped(chi, repeat):
     out = torch.full_like(eng.n2e, 7.0)
     flag = torch.zeros(1, dtype=torch.int32, device=L.device)
     nodes = torch.arange(L.n_nodes, dtype=torch.int32, device=L.device).repeat(repeat)
-    _lib.call("dqz_bp_sweep_k3", L.gptr, chi, eng.T.data_ptr(), eng.n2e.data_ptr(), eng.e2n.data_ptr(),
-              out.data_ptr(), None, src_sel.data_ptr(), None, nodes.data_ptr(), nodes.numel(), flag.data_ptr(),
-              _lib.stream_handle())
+    _lib.call("dqz_bp_sweep_k3", L.gptr, chi, 1, eng.T.data_ptr(), eng.n2e.data_ptr(), eng.e2n.data_ptr(),
+              out.data_ptr(), None, src_sel.data_ptr(), None, nodes.data_ptr(), nodes.numel(), 0, None,
+              flag.data_ptr(), _lib.stream_handle())
     assert int(flag) == 1
     for v in range(L.n_nodes):
         for h in range(L.node_half[v], L.node_half[v] + L.degree[v]):
@@ -98,3 +98,98 @@ def test_other_shapes_are_flagged_and_skipped(chi, repeat):
                 assert float((got - ref).norm() / (ref.norm() * (1 + ref.norm()))) < TOL
             else:
                 assert bool((got == 7.0).all())
+
+
+def uneven_graph(n, dims, phys):
+    """Random 3-regular graph whose bond dimensions cycle through ``dims``."""
+    g = G.get_random_regular_graph(n, 3, phys, 1, 5)
+    for i, e in enumerate(g.edges.values()):
+        e.dimension = dims[i % len(dims)]
+    g.refresh_bond_shapes()
+    return g
+
+
+def positive_messages(eng, gen):
+    L = eng.layout
+    arena = torch.zeros_like(eng.n2e)
+    for h in range(L.n_halves):
+        c = int(L.edge_chi[L.half_edge[h]])
+        a = torch.randn((c, c), dtype=torch.complex128, device="cuda", generator=gen)
+        m = a @ a.mH
+        L.message_view(arena, h).copy_(m / m.diagonal().sum().real)
+    return arena
+
+
+SHAPES = [(10, (16,), 2), (302, (16,), 2), (10, (8,), 2), (1000, (8,), 2),  # uniform: compile-time strides
+          (10, (5,), 2), (160, (12,), 2), (12, (1, 3, 8), 3), (12, (2, 9, 16, 7), 1), (160, (15, 1, 4), 3)]
+
+
+@pytest.mark.parametrize("n,dims,phys", SHAPES)
+def test_padded_sweep_raw_and_change(n, dims, phys):
+    """Messages, unnormalised messages and the largest change, against the generic kernel."""
+    g = uneven_graph(n, dims, phys)
+    eng = engine(g, "flooding")
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    eng.n2e = positive_messages(eng, gen)
+    eng.e2n = positive_messages(eng, gen)
+    ref_n, ref_e = generic_sweep(eng)
+    L = eng.layout
+    shape = L.k3_shape()
+    assert shape == (max(dims), int(dims in ((8,), (16,)) and phys == 2))
+    src_sel, edge_new, _ = eng.topo.device_tables(L.device)
+    nodes = torch.arange(L.n_nodes, dtype=torch.int32, device=L.device)
+    out_n, out_e, raw = (torch.zeros_like(eng.n2e) for _ in range(3))
+    change = torch.zeros(1, dtype=torch.float64, device=L.device)
+    flag = torch.zeros(1, dtype=torch.int32, device=L.device)
+    for n_new, e_new, is_raw, ch in ((out_n, out_e, 0, change), (raw, None, 1, None)):
+        _lib.call("dqz_bp_sweep_k3", L.gptr, *shape, eng.T.data_ptr(), eng.n2e.data_ptr(), eng.e2n.data_ptr(),
+                  n_new.data_ptr(), _lib.ptr(e_new), src_sel.data_ptr(), edge_new.data_ptr(), nodes.data_ptr(),
+                  L.n_nodes, is_raw, _lib.ptr(ch), flag.data_ptr(), _lib.stream_handle())
+    assert int(flag) == 0
+    assert float(change) == pytest.approx(float((out_n - eng.n2e).abs().max()), rel=1e-14)
+    for h in range(L.n_halves):
+        for got, ref in ((out_n, ref_n), (out_e, ref_e)):
+            x, y = L.message_view(got, h), L.message_view(ref, h)
+            assert float((x - y).norm()) < TOL * float(y.norm() * (1 + y.norm()))
+        r = L.message_view(raw, h)
+        assert float((r / r.diagonal().sum() - L.message_view(out_n, h)).norm()) < TOL
+
+
+@pytest.mark.parametrize("n,dims,phys", SHAPES)
+def test_transposed_sweep_matches_generic_adjoint(n, dims, phys):
+    """dqz_bp_vjp_k3 against dqz_bp_node_vjp, both outputs and the fused iterate. A cotangent entry is a few
+    chains of three contractions of at most 2 * 16^3 terms (error about 2e-14 of the norm each, positive
+    messages: no cancellation in the trace): 1e-12 of the arena's norm."""
+    g = uneven_graph(n, dims, phys)
+    eng = engine(g, "flooding")
+    gen = torch.Generator(device="cuda").manual_seed(13)
+    e2n = positive_messages(eng, gen)
+    L = eng.layout
+    cot, add = (torch.randn(L.msg_elems, dtype=torch.complex128, device="cuda", generator=gen) for _ in range(2))
+    nodes = torch.arange(L.n_nodes, dtype=torch.int32, device=L.device)
+    stream = _lib.stream_handle()
+    ref, ref_t = torch.zeros_like(cot), torch.ones_like(eng.T)
+    scratch = torch.empty(_lib.lib().dqz_bp_node_vjp_scratch_bytes(L.n_nodes, L.max_size()), dtype=torch.uint8,
+                          device=L.device)
+    _lib.call("dqz_bp_node_vjp", L.gptr, eng.T.data_ptr(), e2n.data_ptr(), cot.data_ptr(), ref.data_ptr(),
+              ref_t.data_ptr(), nodes.data_ptr(), L.n_nodes, L.max_size(), L.max_chi(), scratch.data_ptr(), stream)
+    shape = L.k3_shape()
+    flag = torch.zeros(1, dtype=torch.int32, device=L.device)
+    own = torch.zeros(L.n_halves, dtype=torch.uint8, device=L.device)
+    raw, got, nxt = (torch.zeros_like(cot) for _ in range(3))
+    got_t = torch.ones_like(eng.T)
+    change = torch.zeros(1, dtype=torch.float64, device=L.device)
+    _lib.call("dqz_bp_sweep_k3", L.gptr, *shape, eng.T.data_ptr(), e2n.data_ptr(), e2n.data_ptr(), raw.data_ptr(),
+              None, own.data_ptr(), None, nodes.data_ptr(), L.n_nodes, 1, None, flag.data_ptr(), stream)
+    for out, ad, ch, tc in ((got, None, None, got_t), (nxt, add, change, None)):
+        _lib.call("dqz_bp_vjp_k3", L.gptr, *shape, eng.T.data_ptr(), e2n.data_ptr(), cot.data_ptr(), raw.data_ptr(),
+                  out.data_ptr(), _lib.ptr(ad), _lib.ptr(ch), _lib.ptr(tc), nodes.data_ptr(), L.n_nodes,
+                  flag.data_ptr(), stream)
+    assert int(flag) == 0
+    assert float((got - ref).norm() / ref.norm()) < 1e-12
+    assert float((got_t - ref_t).norm() / ref_t.norm()) < 1e-12
+    want = add.clone()
+    for h in range(L.n_halves):
+        L.message_view(want, int(L.half_twin[h])).add_(L.message_view(got, h))
+    assert float((nxt - want).norm() / want.norm()) < 1e-14
+    assert float(change) == pytest.approx(float((nxt - cot).abs().max()), rel=1e-14)
