@@ -122,6 +122,7 @@ _SIGNATURES = {
     "dqz_symmetric_gauge": (ctypes.c_int, [_G, _P, _P, _D, _P, _P]),
     "dqz_lambdas_to_messages": (ctypes.c_int, [_G, _P, _P, _P, _I, _P]),
     "dqz_density_matrices": (ctypes.c_int, [_G, _P, _P, _P, _I, _P, _I, _P, _P]),
+    "dqz_density_k3": (ctypes.c_int, [_G, _I, _I, _P, _P, _P, _I, _P, _P, _P]),
     "dqz_density_scratch_bytes": (_S, [_I, _I]),
     "dqz_apply1": (ctypes.c_int, [_G, _P, _P, _P, _I, _P]),
     "dqz_apply_half_gates": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _I, _P]),

@@ -1,0 +1,252 @@
+// Vidal orthogonalisers of one edge (tensor_ops.py:108-130, edge_svd) without
+// message square roots, one warp per edge, bonds up to 16.
+//
+// The reference takes C = sqrt(m_f) sqrt(m_b)^T = U S V^H and the orthogonalisers
+// sqrt(m_f)^-1 U, sqrt(m_b)^-1 conj(V). For positive definite messages any factor
+// m = L L^H serves, since sqrt(m) = L W with W unitary: with Cholesky factors,
+//   C' = L_f^H conj(L_b) = U' S V'^H   (the same S),
+//   G_f = sqrt(m_f)^-1 U = L_f^-H U',  G_b = sqrt(m_b)^-1 conj(V) = conj(L_f U') S^-1,
+// so two Hermitian eigendecompositions and the right singular vectors drop out,
+// leaving two 16-step factorisations, one triangular solve, and a one-sided
+// Jacobi iteration on the columns of C' alone. G_f S G_b^T = 1 holds to rounding
+// by construction; the columns of U' are orthogonal to the Jacobi tolerance
+// relative to their own norms, also for small singular values.
+//
+// The reference drops message eigenvalues up to eps. The factored form is exact
+// only when none are: |G_f|_F^2 = sum 1 / (eigenvalues of m_f) (and the same for
+// b), so both norms below 1 / (2 eps) prove every eigenvalue above 2 eps. Other
+// edges (also those with a pivot up to eps, a null singular value or non-finite
+// entries) are marked and left to the kernel with the eigendecompositions.
+//
+// In the Jacobi rounds four lanes hold a pair of columns in registers (rows sub +
+// 4 i) and the columns move round the circle by shuffles; column norms are
+// carried along the rotations and recomputed every sweep.
+#pragma once
+
+#include "dmma.cuh"
+#include "linalg.cuh"
+
+namespace dqz {
+
+constexpr int ES_MAX = 16, ES_LD = 17;
+constexpr unsigned long long ES_MARK = 0x7ff80000000000e5ull;  // in lambda[0]: edge left to the other kernel
+
+struct EdgeSmem {
+  cd L[2][ES_MAX * ES_LD];  // Cholesky factors, row-major, zero above the diagonal and from bond c on
+  cd X[ES_MAX * ES_LD];     // C', then the unit left singular vectors, column-major
+  double dinv[ES_MAX], s[ES_MAX];
+  int perm[ES_MAX];
+};
+
+__device__ __forceinline__ double quad_sum(double v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+__device__ __forceinline__ cd shfl_cd(cd v, int src) {
+  return mk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+
+// L L^H = (m + m^H) / 2 of both messages at once (lanes 0-15: rows of f, 16-31:
+// rows of b). False when a pivot is not above eps.
+__device__ __forceinline__ bool edge_cholesky(EdgeSmem &S, const cd *mf, const cd *mb, int c, double eps) {
+  const int lane = threadIdx.x & 31, side = lane >> 4, r = lane & 15;
+  for (int i = lane; i < ES_MAX * ES_MAX; i += 32) {
+    const int row = i >> 4, col = i & 15;
+    const bool in = row < c && col < c;
+    S.L[0][row * ES_LD + col] = in ? mf[row * c + col] : czero();
+    S.L[1][row * ES_LD + col] = in ? mb[row * c + col] : czero();
+  }
+  __syncwarp();
+  cd *L = S.L[side];
+  cd A[ES_MAX];
+#pragma unroll
+  for (int k = 0; k < ES_MAX; ++k) {
+    const cd u = L[r * ES_LD + k], l = L[k * ES_LD + r];
+    A[k] = mk(0.5 * (u.x + l.x), 0.5 * (u.y - l.y));
+  }
+  __syncwarp();
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < ES_MAX; ++j) {
+    if (j < c) {
+      const double piv = __shfl_sync(0xffffffffu, A[j].x, (lane & 16) + j);
+      ok = ok && piv > eps;
+      const double inv = rsqrt(piv);
+      const cd l = r > j ? cscale(A[j], inv) : (r == j ? mk(piv * inv, 0.0) : czero());
+      if (r == j && side == 0) S.dinv[j] = inv;
+      L[r * ES_LD + j] = r < c ? l : czero();
+      __syncwarp();
+#pragma unroll
+      for (int k = j + 1; k < ES_MAX; ++k) {
+        const cd lk = cconj(L[k * ES_LD + j]);
+        A[k] = csub(A[k], cmul(l, lk));
+      }
+    } else {
+      L[r * ES_LD + j] = czero();
+    }
+  }
+  __syncwarp();
+  return __all_sync(0xffffffffu, ok);
+}
+
+// One-sided Jacobi on the columns of S.X (c x c): on return S.X holds the unit
+// left singular vectors, S.s the singular values. False when one is numerically
+// null (hestenes' rule).
+__device__ __forceinline__ bool edge_jacobi(EdgeSmem &S, int c) {
+  const int lane = threadIdx.x & 31, grp = lane >> 2, sub = lane & 3;
+  const int np = c + (c & 1), npairs = np / 2;
+  const double tol = 1.1e-16 * sqrt((double)c) * 2.0;
+  const bool seat = grp < npairs;
+  const int ct = grp, cb = np - 1 - grp;  // this group's columns at the start of every sweep
+  cd x[4], y[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    x[i] = seat ? S.X[ct * ES_LD + sub + 4 * i] : czero();
+    y[i] = seat && cb < c ? S.X[cb * ES_LD + sub + 4 * i] : czero();
+  }
+  double al = 0.0, be = 0.0, null_thr = 0.0;
+  for (int sweep = 0; sweep < 60; ++sweep) {
+    al = be = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      al += cabs2(x[i]);
+      be += cabs2(y[i]);
+    }
+    al = quad_sum(al);
+    be = quad_sum(be);
+    if (sweep == 0) null_thr = hestenes_null_scale(c) * warp_sum(sub == 0 ? al + be : 0.0);
+    bool rotated = false;
+    for (int round = 0; round < np - 1; ++round) {
+      cd ga = czero();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) cfmac(ga, x[i], y[i]);
+      ga = mk(quad_sum(ga.x), quad_sum(ga.y));
+      const bool rot = seat && al > null_thr && be > null_thr && cabs2(ga) > tol * tol * al * be;
+      if (__any_sync(0xffffffffu, rot)) {
+        Rot R;
+        if (rot && jacobi_rot(al, be, ga, R)) {
+          rotated = true;
+          // jacobi_rot's J: columns (phase cos, -sin) and (phase sin, cos)
+          const double cs = R.j11.x, sn = -R.j10.x, inv = rsqrt(cabs2(ga));
+          const cd ph = mk(ga.x * inv, ga.y * inv);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const cd p = cmul(x[i], ph), q = y[i];
+            x[i] = mk(cs * p.x - sn * q.x, cs * p.y - sn * q.y);
+            y[i] = mk(sn * p.x + cs * q.x, sn * p.y + cs * q.y);
+          }
+          const double shift = cabs2(ga) * inv * (sn / cs);  // t |ga|
+          al -= shift;
+          be += shift;
+        }
+      }
+      if (npairs > 1) {  // next round: first column fixed, the others one seat round the circle
+        const int up = lane - 4, down = lane + 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const cd from_up = shfl_cd(grp == 0 ? y[i] : x[i], up & 31);
+          const cd from_down = shfl_cd(y[i], down & 31);
+          const cd keep = x[i];
+          if (grp > 0) x[i] = from_up;
+          y[i] = grp == npairs - 1 ? keep : from_down;
+        }
+        const double a_up = __shfl_sync(0xffffffffu, grp == 0 ? be : al, up & 31);
+        const double b_down = __shfl_sync(0xffffffffu, be, down & 31);
+        const double keep = al;
+        if (grp > 0) al = a_up;
+        be = grp == npairs - 1 ? keep : b_down;
+      }
+    }
+    if (!__any_sync(0xffffffffu, rotated)) break;
+  }
+  al = be = 0.0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    al += cabs2(x[i]);
+    be += cabs2(y[i]);
+  }
+  al = quad_sum(al);
+  be = quad_sum(be);
+  const bool two = seat && cb < c;
+  const double sa = sqrt(al), sb = sqrt(be), ia = 1.0 / sa, ib = 1.0 / sb;
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (seat) S.X[ct * ES_LD + sub + 4 * i] = cscale(x[i], ia);
+    if (two) S.X[cb * ES_LD + sub + 4 * i] = cscale(y[i], ib);
+  }
+  if (seat && sub == 0) {
+    S.s[ct] = sa;
+    if (two) S.s[cb] = sb;
+  }
+  __syncwarp();
+  return __all_sync(0xffffffffu, (!seat || al > null_thr) && (!two || be > null_thr));
+}
+
+// One edge by the factored form; false (nothing written but possibly
+// orthogonalisers, which the other kernel overwrites) when it does not apply.
+__device__ __forceinline__ bool edge_svd_factored(EdgeSmem &S, const cd *mf, const cd *mb, int c, double eps, cd *Gf,
+                                                  cd *Gb, double *lam) {
+  const int lane = threadIdx.x & 31;
+  if (!edge_cholesky(S, mf, mb, c, eps)) return false;
+  CTile<2, 2> t;
+  t.clear();
+  cgemm<true, true, 2>(
+      t, [&](int i, int k) { return S.L[0][k * ES_LD + i]; }, [&](int k, int j) { return S.L[1][k * ES_LD + j]; });
+  ctile_each(t, [&](int i, int j, cd v) { S.X[j * ES_LD + i] = v; });
+  __syncwarp();
+  if (!edge_jacobi(S, c)) return false;
+  warp_sort_desc(S.s, c, S.perm);
+  const double sj = lane < c ? S.s[S.perm[lane]] : 0.0;
+  const double l0 = sj / sqrt(warp_sum(sj * sj));
+  const double kept = l0 > eps ? l0 : 0.0;
+  const unsigned mask = __ballot_sync(0xffffffffu, lane < c && kept > eps);
+  const double scale = 1.0 / sqrt((double)__popc(mask));
+  // G_b = conj(L_f U') / s, columns in descending order
+  t.clear();
+  cgemm<false, false, 2>(
+      t, [&](int i, int k) { return S.L[0][i * ES_LD + k]; },
+      [&](int k, int j) { return j < c ? S.X[S.perm[j] * ES_LD + k] : czero(); });
+  double nb = 0.0;
+  ctile_each(t, [&](int i, int j, cd v) {
+    if (i >= c || j >= c) return;
+    const cd x = cscale(cconj(v), 1.0 / S.s[S.perm[j]]);
+    nb += cabs2(x);
+    Gb[i * c + j] = (mask >> j) & 1u ? cscale(x, scale) : czero();
+  });
+  nb = warp_sum(nb);
+  // G_f = L_f^-H U': lane (half, j) holds the rows of parity `half` of column j
+  const int j = lane & 15, half = lane >> 4;
+  cd u[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) u[k] = j < c ? S.X[S.perm[j] * ES_LD + 2 * k + half] : czero();
+#pragma unroll
+  for (int i = ES_MAX - 1; i >= 0; --i) {
+    if (i < c) {
+      const cd xi = cscale(shfl_cd(u[i >> 1], j + 16 * (i & 1)), S.dinv[i]);
+      if (half == (i & 1)) u[i >> 1] = xi;
+#pragma unroll
+      for (int k = 0; k < (i + 1) / 2; ++k) {
+        const int row = 2 * k + half;
+        const cd l = row < i ? S.L[0][i * ES_LD + row] : czero();
+        u[k] = csub(u[k], cmulc(l, xi));
+      }
+    }
+  }
+  double nf = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int row = 2 * k + half;
+    if (j < c && row < c) {
+      nf += cabs2(u[k]);
+      Gf[row * c + j] = (mask >> j) & 1u ? cscale(u[k], scale) : czero();
+    }
+  }
+  nf = warp_sum(nf);
+  const double limit = 0.5 / eps;
+  if (!(nf < limit) || !(nb < limit)) return false;
+  if (lane < c) lam[lane] = kept;
+  return true;
+}
+
+}  // namespace dqz

@@ -1,6 +1,7 @@
 // Gauge kernels (FP64 / complex128):
 //  * vidal_edges    -- tensor_ops.py:108-130 (edge_svd): one warp per edge for
-//                      chi <= 16, one CTA per edge above
+//                      chi <= 16 (by Cholesky factors where they apply, then the
+//                      marked edges by eigendecompositions), one CTA per edge above
 //  * absorb         -- tensor_ops.py:88-93 (absorb_by_node), one CTA per node
 //  * vidal_distance -- tensor_ops.py:143-175 + mappings/vidal_distance.py:17-42:
 //                      one warp per half-edge for chi <= 16, one CTA per
@@ -10,7 +11,9 @@
 //  * symmetric      -- tensor_ops.py:189-199 (canonicalize)
 //  * lambdas->msgs  -- mappings/symmetric_gauge.py:50-61
 //  * density        -- mappings/density_matrix.py:16-37
+#include "edge_svd.cuh"
 #include "linalg.cuh"
+#include "trace_norm.cuh"
 
 using namespace dqz;
 
@@ -149,8 +152,34 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_edges_kernel(dqz_graph_t 
   }
 }
 
-// One warp per edge (chi <= WARP_MAX_CHI): the same steps as
-// vidal_edges_kernel on the warp's own slice of shared memory.
+// One warp per edge (chi <= WARP_MAX_CHI), the factored form (edge_svd.cuh);
+// edges it does not cover get ES_MARK in lambda[0]. Measured at 1,536 edges of
+// bond 16 (random 3-regular graph, 1,024 nodes): 116 us, 1,442 us with the
+// eigendecompositions.
+constexpr int ES_WARPS = 4;
+__global__ void __launch_bounds__(32 * ES_WARPS, 4) vidal_edges_factored_kernel(dqz_graph_t g,
+                                                                                 const cd *__restrict__ n2e,
+                                                                                 double eps, cd *orth,
+                                                                                 double *lambdas, int max_chi,
+                                                                                 const int32_t *__restrict__ sel,
+                                                                                 int total) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  EdgeSmem &S = reinterpret_cast<EdgeSmem *>(smem_raw)[threadIdx.x >> 5];
+  for (int it = blockIdx.x * ES_WARPS + (threadIdx.x >> 5); it < total; it += gridDim.x * ES_WARPS) {
+    const int e = sel ? sel[it] : it;
+    const int c = g.edge_chi[e];
+    double *lam = lambdas + g.edge_lam_off[e];
+    const long long of = g.half_msg_off[g.edge_half[2 * e]], ob = g.half_msg_off[g.edge_half[2 * e + 1]];
+    const bool fits = c <= max_chi;  // else the caller's max_chi is below this bond: flag it
+    const bool done = fits && edge_svd_factored(S, n2e + of, n2e + ob, c, eps, orth + of, orth + ob, lam);
+    if (!done && (threadIdx.x & 31) == 0)
+      lam[0] = __longlong_as_double((long long)(fits ? ES_MARK : 0x7ff8000000000000ull));
+    __syncwarp();
+  }
+}
+
+// The marked edges, one warp each: the same steps as vidal_edges_kernel on the
+// warp's own slice of shared memory.
 __host__ __device__ inline size_t warp_edge_bytes(int c) {
   return round16(WARP_ROTS * sizeof(Rot)) + round16(vidal_edge_bytes(c));
 }
@@ -176,10 +205,10 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_edges_warp_kernel(dqz_gra
     const int h0 = g.edge_half[2 * e], h1 = g.edge_half[2 * e + 1];
     const int c = g.edge_chi[e];
     double *lam = lambdas + g.edge_lam_off[e];
-    if (c > max_chi) {  // the caller's max_chi is below this bond: flag it
-      if (lane == 0) lam[0] = __longlong_as_double(0x7ff8000000000000ll);
-      continue;
-    }
+    // the factored kernel before this one did every edge it did not mark
+    const unsigned long long mark = (unsigned long long)__double_as_longlong(lam[0]);
+    __syncwarp();
+    if (mark != ES_MARK) continue;
     const cd *mf = n2e + g.half_msg_off[h0];
     const cd *mb = n2e + g.half_msg_off[h1];
     for (int i = lane; i < c * c; i += 32) {
@@ -571,35 +600,105 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_distance_kernel(dqz_graph
   }
 }
 
-// One warp per half-edge (chi <= WARP_MAX_CHI). The bond slice is streamed
-// through the warp's shared memory in chunks of VD_CHUNK rows as
-// Y[x][a] = T[.., a@e, ..](x) * prod_{f != e} lambda_f[idx_f(x)], so that
-// R = Y^H Y (the lambda^2-weighted reduced matrix) reads every tensor entry
-// from L2 once; each lane accumulates up to VD_PAIRS entries (a' <= a) of R
-// from the staged rows, and the trace norm comes from warp_herm_eigh.
+// One warp per half-edge (chi <= WARP_MAX_CHI). R[a'][a] = sum_x conj(T[x, a'])
+// T[x, a] prod_{f != e} lambda_f[idx_f(x)]^2 (the lambda^2-weighted reduced
+// matrix) is accumulated on the FP64 tensor cores straight from global memory:
+// every entry of T is used once per half-edge, and the A fragment (conjugated)
+// and the B fragment (times the weight) of a step are the same loads. The rows x
+// go 32 at a time, each lane decomposing one of them into its offset and weight;
+// only the tiles on and above the diagonal are formed. The trace norm then comes
+// from warp_trace_norm. Measured at 3,072 half-edges of bond 16: 231 us, 980 us
+// with register-accumulated entries and a Jacobi iteration.
 constexpr int VD_CHUNK = 32;
-constexpr int VD_PAIRS = (WARP_MAX_CHI * (WARP_MAX_CHI + 1) / 2 + 31) / 32;
+constexpr int VD_LD = 17;
 
-__host__ __device__ inline size_t warp_vd_bytes(int c) {
-  return round16(WARP_ROTS * sizeof(Rot)) + round16((size_t)c * c * sizeof(cd)) + round16((size_t)c * sizeof(double)) +
-         round16(VD_CHUNK * sizeof(double)) + round16((size_t)VD_CHUNK * c * sizeof(cd));
+struct VdSmem {
+  cd R[WARP_MAX_CHI * VD_LD];
+  TraceNormSmem tn;
+  double w[VD_CHUNK];
+  long long off[VD_CHUNK];
+};
+
+// R of one half-edge into S.R (rows / columns below 8 TN).
+template <int TN>
+__device__ __forceinline__ void vd_gram(const cd *__restrict__ T, const NodeShape &s, int e,
+                                        const dqz_graph_t &g, const double *__restrict__ lambdas, VdSmem &S) {
+  const int lane = threadIdx.x & 31, row = lane >> 2, q = lane & 3;
+  const int ce = s.dims[e], Re = (int)s.stride[e], P = (int)(s.size / ce);
+  double re[TN][TN][2], im[TN][TN][2];
+#pragma unroll
+  for (int r = 0; r < TN; ++r)
+#pragma unroll
+    for (int n = 0; n < TN; ++n) re[r][n][0] = re[r][n][1] = im[r][n][0] = im[r][n][1] = 0.0;
+  for (int x0 = 0; x0 < P; x0 += VD_CHUNK) {
+    __syncwarp();
+    const int x = x0 + lane;
+    double wt = 0.0;
+    long long o0 = 0;
+    if (x < P) {
+      const int l = x / Re, r = x - l * Re;
+      o0 = (long long)l * ce * Re + r;  // offset with a_e = 0
+      wt = 1.0;
+      for (int f = 0; f < s.k; ++f) {
+        if (f == e) continue;
+        const int idx = ((int)o0 / (int)s.stride[f]) % s.dims[f];
+        const double lf = lambdas[g.edge_lam_off[g.half_edge[s.half0 + f]] + idx];
+        wt *= lf * lf;
+      }
+    }
+    S.w[lane] = wt;
+    S.off[lane] = o0;
+    __syncwarp();
+    // loads of half a chunk in flight before its products
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      cd t[4][TN];
+      double w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int xl = 16 * h + 4 * k + q;
+        const cd *src = T + S.off[xl];
+        w[k] = S.w[xl];
+#pragma unroll
+        for (int r = 0; r < TN; ++r) {
+          const int a = 8 * r + row;
+          t[k][r] = a < ce ? src[(long long)a * Re] : czero();
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int n = 0; n < TN; ++n) {
+          const cd bn = cscale(t[k][n], w[k]);
+#pragma unroll
+          for (int r = 0; r <= n; ++r) {  // conj(t_r) bn
+            dmma(re[r][n], t[k][r].x, bn.x);
+            dmma(im[r][n], t[k][r].x, bn.y);
+            dmma(re[r][n], t[k][r].y, bn.y);
+            dmma(im[r][n], -t[k][r].y, bn.x);
+          }
+        }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < TN; ++r)
+#pragma unroll
+    for (int n = r; n < TN; ++n)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int a1 = 8 * r + row, a2 = 8 * n + 2 * q + i;
+        S.R[a1 * VD_LD + a2] = mk(re[r][n][i], im[r][n][i]);
+        if (r < n) S.R[a2 * VD_LD + a1] = mk(re[r][n][i], -im[r][n][i]);
+      }
+  __syncwarp();
 }
 
-__global__ void __launch_bounds__(GAUGE_THREADS, 3) vidal_distance_warp_kernel(
+__global__ void __launch_bounds__(GAUGE_THREADS) vidal_distance_warp_kernel(
     dqz_graph_t g, const cd *__restrict__ Tall, const double *__restrict__ lambdas, double eps, double *partial,
     int max_chi, const int32_t *__restrict__ sel, int n_sel) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  unsigned char *wbase = smem_raw + (size_t)wid * warp_vd_bytes(max_chi);
-  Rot *rots = reinterpret_cast<Rot *>(wbase);
-  unsigned char *q = wbase + round16(WARP_ROTS * sizeof(Rot));
-  cd *Rm = reinterpret_cast<cd *>(q);
-  q += round16((size_t)max_chi * max_chi * sizeof(cd));
-  double *wv = reinterpret_cast<double *>(q);
-  q += round16((size_t)max_chi * sizeof(double));
-  double *wl = reinterpret_cast<double *>(q);
-  q += round16(VD_CHUNK * sizeof(double));
-  cd *Ys = reinterpret_cast<cd *>(q);
+  VdSmem &S = reinterpret_cast<VdSmem *>(smem_raw)[wid];
   const int total = sel ? n_sel : g.n_halves;
   for (int it = blockIdx.x * wpb + wid; it < total; it += gridDim.x * wpb) {
     const int h = sel ? sel[it] : it;
@@ -612,77 +711,26 @@ __global__ void __launch_bounds__(GAUGE_THREADS, 3) vidal_distance_warp_kernel(
       if (lane == 0) partial[h] = __longlong_as_double(0x7ff8000000000000ll);
       continue;
     }
-    const int P = (int)(s.size / ce), Re = (int)s.stride[e];
     const cd *T = Tall + g.node_off[v];
-    const int npair = ce * (ce + 1) / 2;
-    int pa[VD_PAIRS], pb[VD_PAIRS];
-    cd acc[VD_PAIRS];
-#pragma unroll
-    for (int j = 0; j < VD_PAIRS; ++j) {
-      const int pi = lane + 32 * j;
-      pa[j] = -1;
-      pb[j] = 0;
-      acc[j] = czero();
-      if (pi < npair) {
-        int ap = 0, rem = pi;
-        while (rem >= ce - ap) {
-          rem -= ce - ap;
-          ++ap;
-        }
-        pa[j] = ap;
-        pb[j] = ap + rem;
-      }
-    }
-    for (int x0 = 0; x0 < P; x0 += VD_CHUNK) {
-      const int nx = P - x0 < VD_CHUNK ? P - x0 : VD_CHUNK;
-      if (lane < nx) {  // lambda weight (not squared) of row x0 + lane
-        const int x = x0 + lane, l = x / Re, r = x - l * Re;
-        const int o0 = l * ce * Re + r;  // offset with a_e = 0
-        double wt = 1.0;
-        for (int f = 0; f < s.k; ++f) {
-          if (f == e) continue;
-          const int idx = (o0 / (int)s.stride[f]) % s.dims[f];
-          wt *= lambdas[g.edge_lam_off[g.half_edge[s.half0 + f]] + idx];
-        }
-        wl[lane] = wt;
-      }
-      __syncwarp();
-      for (int t = lane; t < nx * ce; t += 32) {  // rows x fastest across lanes
-        const int a = t / nx, jx = t - a * nx;
-        const int x = x0 + jx, l = x / Re, r = x - l * Re;
-        Ys[jx * ce + a] = cscale(T[(long long)(l * ce + a) * Re + r], wl[jx]);
-      }
-      __syncwarp();
-      for (int jx = 0; jx < nx; ++jx) {
-        const cd *row = Ys + jx * ce;
-#pragma unroll
-        for (int j = 0; j < VD_PAIRS; ++j)
-          if (pa[j] >= 0) cfmac(acc[j], row[pa[j]], row[pb[j]]);
-      }
-      __syncwarp();
-    }
-#pragma unroll
-    for (int j = 0; j < VD_PAIRS; ++j)
-      if (pa[j] >= 0) {
-        Rm[pa[j] * ce + pb[j]] = acc[j];
-        Rm[pb[j] * ce + pa[j]] = cconj(acc[j]);
-      }
-    __syncwarp();
+    if (ce <= 8)
+      vd_gram<1>(T, s, e, g, lambdas, S);
+    else
+      vd_gram<2>(T, s, e, g, lambdas, S);
+    cd *Rm = S.R;
     cd tr = czero();
-    for (int i = 0; i < ce; ++i) tr = cadd(tr, Rm[i * ce + i]);
+    for (int i = 0; i < ce; ++i) tr = cadd(tr, Rm[i * VD_LD + i]);
     int cnt = 0;
-    for (int i = 0; i < ce; ++i) cnt += cdiv(Rm[i * ce + i], tr).x > eps ? 1 : 0;
-    __syncwarp();
-    for (int i = lane; i < ce * ce; i += 32) Rm[i] = cdiv(Rm[i], tr);
+    for (int i = 0; i < ce; ++i) cnt += cdiv(Rm[i * VD_LD + i], tr).x > eps ? 1 : 0;
     __syncwarp();
     const double idv = 1.0 / (double)cnt;
-    for (int i = lane; i < ce; i += 32)
-      if (Rm[i * ce + i].x > eps) Rm[i * ce + i].x -= idv;
+    for (int i = lane; i < ce * ce; i += 32) {
+      const int a1 = i / ce, a2 = i % ce;
+      cd x = cdiv(Rm[a1 * VD_LD + a2], tr);
+      if (a1 == a2 && x.x > eps) x.x -= idv;
+      Rm[a1 * VD_LD + a2] = x;
+    }
     __syncwarp();
-    warp_herm_eigh(Rm, ce, nullptr, 0, ce, wv, rots);
-    double t = 0.0;
-    for (int i = lane; i < ce; i += 32) t += fabs(wv[i]);
-    t = warp_sum(t);
+    const double t = warp_trace_norm(Rm, VD_LD, ce, S.tn);
     if (lane == 0) partial[h] = t;
     __syncwarp();
   }
@@ -815,6 +863,10 @@ extern "C" int dqz_vidal_edges(const dqz_graph_t *g, const void *n2e, double eps
     wpb = wpb < 1 ? 1 : (wpb > GAUGE_THREADS / 32 ? GAUGE_THREADS / 32 : wpb);
     const int tuned = dqz_get_tuning(DQZ_TUNE_GAUGE_EDGE_WARPS);
     if (tuned > 0 && (size_t)tuned * per <= SMEM_LIMIT) wpb = tuned;
+    DQZ_SMEM_ATTR_ONCE(vidal_edges_factored_kernel, SMEM_LIMIT);
+    vidal_edges_factored_kernel<<<(total + ES_WARPS - 1) / ES_WARPS, 32 * ES_WARPS, ES_WARPS * sizeof(EdgeSmem),
+                                  stream>>>(*g, (const cd *)n2e, eps, (cd *)orth, lambdas, max_chi, edges, total);
+    DQZ_CHECK_LAUNCH();
     DQZ_SMEM_ATTR_ONCE(vidal_edges_warp_kernel, SMEM_LIMIT);
     vidal_edges_warp_kernel<<<(total + wpb - 1) / wpb, 32 * wpb, wpb * per, stream>>>(
         *g, (const cd *)n2e, eps, (cd *)orth, lambdas, max_chi, edges, total);
@@ -895,9 +947,8 @@ extern "C" int dqz_vidal_distance(const dqz_graph_t *g, const void *tensors, con
   const int total = halves ? n_sel : nh;
   if (total > 0) {
     if (max_chi <= WARP_MAX_CHI && dqz_get_tuning(DQZ_TUNE_GAUGE_PATH) != 2) {
-      const size_t per = warp_vd_bytes(max_chi);
-      int wpb = (int)(WARP_BLOCK_SMEM / per);
-      wpb = wpb < 1 ? 1 : (wpb > GAUGE_THREADS / 32 ? GAUGE_THREADS / 32 : wpb);
+      const size_t per = sizeof(VdSmem);
+      int wpb = 4;
       const int tuned = dqz_get_tuning(DQZ_TUNE_GAUGE_DIST_WARPS);
       if (tuned > 0 && (size_t)tuned * per <= SMEM_LIMIT) wpb = tuned;
       DQZ_SMEM_ATTR_ONCE(vidal_distance_warp_kernel, SMEM_LIMIT);

@@ -366,6 +366,11 @@ int dqz_density_matrices(const dqz_graph_t *g, const void *tensors, const void *
                          const int32_t *nodes, int32_t n_nodes, void *rho,
                          int32_t max_size, void *scratch, cudaStream_t stream);
 size_t dqz_density_scratch_bytes(int32_t n_nodes, int32_t max_size);
+/* The same for degree-3 nodes with bonds up to 16 on the FP64 tensor cores
+ * (max_chi, uniform and *error_flag as dqz_bp_sweep_k3); needs no scratch. */
+int dqz_density_k3(const dqz_graph_t *g, int32_t max_chi, int32_t uniform, const void *tensors,
+                   const void *e2n, const int32_t *nodes, int32_t n_nodes, void *rho,
+                   int32_t *error_flag, cudaStream_t stream);
 
 /* ---- Gates (tensor_graph.py:268-446, tensor_ops.py:202-389) --------------- */
 
