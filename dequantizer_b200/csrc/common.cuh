@@ -43,6 +43,29 @@ __device__ __forceinline__ cd cdiv(cd a, cd b) {
   return mk((a.x * b.x + a.y * b.y) / den, (a.y * b.x - a.x * b.y) / den);
 }
 
+// ------------------------------------------------- reciprocals and roots
+// 1 / sqrt(x) and 1 / x for finite x in [1e-290, 1e290], within 2 ulp (largest
+// relative difference from CUDA's 2.7e-16 and 2.2e-16 over 2.6e8 values): the PTX
+// approximations (rsqrt.approx / rcp.approx.ftz.f64, about 20 bits) and one
+// third-order step of Householder's iteration (The Numerical Treatment of a
+// Single Nonlinear Equation, 1970): with e = 1 - x y^2, y (1 + e / 2 + 3 e^2 / 8);
+// with e = 1 - x y, y (1 + e + e^2). Four dependent multiply-adds after the
+// seed: a Jacobi rotation or a Householder reflector is a chain of these on
+// every lane.
+__device__ __forceinline__ double fast_rsqrt(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double fast_rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y * e, 1.0 + e, y);
+}
+__device__ __forceinline__ bool fast_range(double x) { return x >= 1e-290 && x <= 1e290; }
+
 // ------------------------------------------------------------- reductions
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

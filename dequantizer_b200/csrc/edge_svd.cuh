@@ -19,12 +19,11 @@
 // entries) are marked and left to the kernel with the eigendecompositions.
 //
 // In the Jacobi rounds four lanes hold a pair of columns in registers (rows sub +
-// 4 i) and the columns move round the circle by shuffles; column norms are
-// carried along the rotations and recomputed every sweep.
+// 4 i) and the columns move to their next seats by shuffles (as reg_jacobi).
 #pragma once
 
 #include "dmma.cuh"
-#include "linalg.cuh"
+#include "reg_linalg.cuh"
 
 namespace dqz {
 
@@ -71,7 +70,7 @@ __device__ __forceinline__ bool edge_cholesky(EdgeSmem &S, const cd *mf, const c
     if (j < c) {
       const double piv = __shfl_sync(0xffffffffu, A[j].x, (lane & 16) + j);
       ok = ok && piv > eps;
-      const double inv = rsqrt(piv);
+      const double inv = fast_rsqrt(piv);  // piv > eps, or the edge is given up
       const cd l = r > j ? cscale(A[j], inv) : (r == j ? mk(piv * inv, 0.0) : czero());
       if (r == j && side == 0) S.dinv[j] = inv;
       L[r * ES_LD + j] = r < c ? l : czero();
@@ -96,91 +95,64 @@ __device__ __forceinline__ bool edge_jacobi(EdgeSmem &S, int c) {
   const int lane = threadIdx.x & 31, grp = lane >> 2, sub = lane & 3;
   const int np = c + (c & 1), npairs = np / 2;
   const double tol = 1.1e-16 * sqrt((double)c) * 2.0;
-  const bool seat = grp < npairs;
-  const int ct = grp, cb = np - 1 - grp;  // this group's columns at the start of every sweep
+  const bool seat = grp < npairs, last = grp == npairs - 1;
+  const int ct = grp == 0 ? 0 : grp + 1, cb = grp == 0 ? 1 : np - grp;  // rr_pair's step 0
+  const bool has_x = seat && ct < c, has_y = seat && cb < c;
   cd x[4], y[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    x[i] = seat ? S.X[ct * ES_LD + sub + 4 * i] : czero();
-    y[i] = seat && cb < c ? S.X[cb * ES_LD + sub + 4 * i] : czero();
+    x[i] = has_x ? S.X[ct * ES_LD + sub + 4 * i] : czero();
+    y[i] = has_y ? S.X[cb * ES_LD + sub + 4 * i] : czero();
   }
-  double al = 0.0, be = 0.0, null_thr = 0.0;
+  double al, be;
+  cd ga;
+  pair_products(x, y, ga, al, be);
+  const double null_thr = hestenes_null_scale(c) * warp_sum(al + be);
   for (int sweep = 0; sweep < 60; ++sweep) {
-    al = be = 0.0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      al += cabs2(x[i]);
-      be += cabs2(y[i]);
-    }
-    al = quad_sum(al);
-    be = quad_sum(be);
-    if (sweep == 0) null_thr = hestenes_null_scale(c) * warp_sum(sub == 0 ? al + be : 0.0);
     bool rotated = false;
     for (int round = 0; round < np - 1; ++round) {
-      cd ga = czero();
-#pragma unroll
-      for (int i = 0; i < 4; ++i) cfmac(ga, x[i], y[i]);
+      pair_products(x, y, ga, al, be);
       ga = mk(quad_sum(ga.x), quad_sum(ga.y));
+      al = quad_sum(al);
+      be = quad_sum(be);
       const bool rot = seat && al > null_thr && be > null_thr && cabs2(ga) > tol * tol * al * be;
-      if (__any_sync(0xffffffffu, rot)) {
-        Rot R;
-        if (rot && jacobi_rot(al, be, ga, R)) {
-          rotated = true;
-          // jacobi_rot's J: columns (phase cos, -sin) and (phase sin, cos)
-          const double cs = R.j11.x, sn = -R.j10.x, inv = rsqrt(cabs2(ga));
-          const cd ph = mk(ga.x * inv, ga.y * inv);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const cd p = cmul(x[i], ph), q = y[i];
-            x[i] = mk(cs * p.x - sn * q.x, cs * p.y - sn * q.y);
-            y[i] = mk(sn * p.x + cs * q.x, sn * p.y + cs * q.y);
-          }
-          const double shift = cabs2(ga) * inv * (sn / cs);  // t |ga|
-          al -= shift;
-          be += shift;
-        }
-      }
-      if (npairs > 1) {  // next round: first column fixed, the others one seat round the circle
-        const int up = lane - 4, down = lane + 4;
+      PhaseRot R;
+      if (rot && phase_rot(al, be, ga, R)) {
+        rotated = true;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const cd from_up = shfl_cd(grp == 0 ? y[i] : x[i], up & 31);
-          const cd from_down = shfl_cd(y[i], down & 31);
-          const cd keep = x[i];
-          if (grp > 0) x[i] = from_up;
-          y[i] = grp == npairs - 1 ? keep : from_down;
+          const cd p = cmul(x[i], R.ph), q = y[i];
+          x[i] = mk(R.cs * p.x - R.sn * q.x, R.cs * p.y - R.sn * q.y);
+          y[i] = mk(R.sn * p.x + R.cs * q.x, R.sn * p.y + R.cs * q.y);
         }
-        const double a_up = __shfl_sync(0xffffffffu, grp == 0 ? be : al, up & 31);
-        const double b_down = __shfl_sync(0xffffffffu, be, down & 31);
-        const double keep = al;
-        if (grp > 0) al = a_up;
-        be = grp == npairs - 1 ? keep : b_down;
+      }
+      if (npairs > 1) {  // upper columns one seat down (seat 1's to seat 0's lower place), lower ones one up
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const cd nx = shfl_cd(x[i], (lane + 4) & 31), ny = shfl_cd(y[i], (lane - 4) & 31), ky = y[i];
+          y[i] = grp == 0 ? nx : ny;
+          if (grp > 0) x[i] = last ? ky : nx;
+        }
       }
     }
     if (!__any_sync(0xffffffffu, rotated)) break;
   }
-  al = be = 0.0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    al += cabs2(x[i]);
-    be += cabs2(y[i]);
-  }
+  pair_products(x, y, ga, al, be);
   al = quad_sum(al);
   be = quad_sum(be);
-  const bool two = seat && cb < c;
   const double sa = sqrt(al), sb = sqrt(be), ia = 1.0 / sa, ib = 1.0 / sb;
   __syncwarp();
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    if (seat) S.X[ct * ES_LD + sub + 4 * i] = cscale(x[i], ia);
-    if (two) S.X[cb * ES_LD + sub + 4 * i] = cscale(y[i], ib);
+    if (has_x) S.X[ct * ES_LD + sub + 4 * i] = cscale(x[i], ia);
+    if (has_y) S.X[cb * ES_LD + sub + 4 * i] = cscale(y[i], ib);
   }
-  if (seat && sub == 0) {
-    S.s[ct] = sa;
-    if (two) S.s[cb] = sb;
+  if (sub == 0) {
+    if (has_x) S.s[ct] = sa;
+    if (has_y) S.s[cb] = sb;
   }
   __syncwarp();
-  return __all_sync(0xffffffffu, (!seat || al > null_thr) && (!two || be > null_thr));
+  return __all_sync(0xffffffffu, (!has_x || al > null_thr) && (!has_y || be > null_thr));
 }
 
 // One edge by the factored form; false (nothing written but possibly

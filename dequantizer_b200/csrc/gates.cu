@@ -6,19 +6,27 @@
 #include <cooperative_groups.h>
 
 #include "linalg.cuh"
+#include "su.cuh"
 
 using namespace dqz;
+
+namespace dqz {
+// su_reg.cu: jobs whose factors fit the registers of a CTA
+size_t su_reg_scratch_bytes(int n, int max_rows);
+int su_reg(const dqz_graph_t *g, void *tensors, double *lambdas, const int32_t *edges, const uint8_t *ctrl_is_first,
+           const void *halves, const int32_t *ranks, int n, double eps, int max_rank, int max_rows, double *err,
+           double *entropy, uint8_t *done, void *ws, size_t ws_bytes, cudaStream_t stream);
+}  // namespace dqz
 
 namespace {
 
 constexpr int GATE_THREADS = 256;
 constexpr size_t SMEM_LIMIT = 200 * 1024;
-const double F32_MAX = 3.4028234663852886e38;
-constexpr int HALF_STRIDE = 4 * DQZ_MAX_PHYS * DQZ_MAX_PHYS;  // complex entries per gate half
+constexpr int HALF_STRIDE = SU_HALF_STRIDE;
 constexpr int SHAPE_ROW = DQZ_MAX_DEGREE + 4;                 // k, d, slot, r, dims...
 
-__device__ __forceinline__ double safe_inverse(double l, double eps) { return 1.0 / ((l < eps ? F32_MAX : 0.0) + l); }
-__device__ __forceinline__ double safe_truncate(double l, double eps) { return l > eps ? l : 0.0; }
+__device__ __forceinline__ double safe_inverse(double l, double eps) { return su_safe_inverse(l, eps); }
+__device__ __forceinline__ double safe_truncate(double l, double eps) { return su_safe_truncate(l, eps); }
 
 // ------------------------------------------------------------------ apply1
 __global__ void __launch_bounds__(GATE_THREADS) apply1_kernel(dqz_graph_t g, cd *Tall, const int32_t *nodes,
@@ -109,30 +117,6 @@ __global__ void __launch_bounds__(GATE_THREADS) half_gates_kernel(const cd *Tin,
 }
 
 // ----------------------------------------------------------- simple update
-struct SUSide {
-  int node, slot, k, d, half0;
-  int dims[DQZ_MAX_DEGREE];
-  long long stride[DQZ_MAX_DEGREE];
-  const double *lam[DQZ_MAX_DEGREE];
-  int M;  // rows: d * prod_{f != slot} dims
-};
-
-__device__ void su_load_side(const dqz_graph_t &g, const double *lambdas, int h, SUSide &S) {
-  S.node = g.half_node[h];
-  NodeShape s;
-  load_shape(g, S.node, s);
-  S.k = s.k;
-  S.d = s.d;
-  S.half0 = s.half0;
-  S.slot = h - s.half0;
-  for (int f = 0; f < s.k; ++f) {
-    S.dims[f] = s.dims[f];
-    S.stride[f] = s.stride[f];
-    S.lam[f] = lambdas + g.edge_lam_off[g.half_edge[s.half0 + f]];
-  }
-  S.M = (int)(s.size / s.dims[S.slot]);
-}
-
 // Decompose row R = (other bonds in order, o): returns the tensor offset
 // without the slot bond and the physical index, and the product of
 // lambda weights (or of their safe inverses).
@@ -219,31 +203,7 @@ __device__ void su_write(const SUSide &S, const cd *X, int rank, cd *T, double e
 // per SM; the on-chip form takes the larger ones that fit.
 constexpr int SUF_MIN_ROWS = 256;
 
-// Dimensions of one side of a job in the shared-memory form (below):
-//   B = lambda-weighted node tensor, rows b (the other bonds), columns (a, i)
-//       (updated bond, physical index): MB x KB;
-//   S = R_B with the half gate applied, rows (c, o), columns (a, rho): MS x KS;
-//   muB / muS = min(rows, columns): reflector counts, rows of R.
-struct SufDims {
-  int MB, KB, muB, MS, KS, muS;
-};
-
-__device__ __forceinline__ void suf_dims(const SUSide &S, int r, SufDims &D) {
-  const int ce = S.dims[S.slot];
-  D.MB = S.M / S.d;
-  D.KB = ce * S.d;
-  D.muB = D.MB < D.KB ? D.MB : D.KB;
-  D.MS = D.muB * S.d;
-  D.KS = ce * r;
-  D.muS = D.MS < D.KS ? D.MS : D.KS;
-}
-
 __host__ __device__ __forceinline__ long long suf_even(long long x) { return (x + 1) & ~1ll; }
-
-// Largest kept rank of a job: max_rank when it cuts below K = KS, else K.
-__host__ __device__ __forceinline__ int suf_rank_bound(int K, int max_rank) {
-  return (max_rank > 0 && max_rank < K) ? max_rank : K;
-}
 
 // Size of the combined core | W region: the core SVD needs 2 K^2; later the
 // same space holds V^H V (muB^2) and then V^H Z (muB x d*rank).
@@ -780,7 +740,9 @@ extern "C" size_t dqz_simple_update_scratch_bytes(int32_t n, int32_t max_rows, i
   const size_t cluster = (max_rows >= SUF_MIN_ROWS && n > 0)
                              ? (size_t)2 * su_cluster_pairs(n) * su_cluster_cap(max_rows, max_cols) * sizeof(cd)
                              : 0;
-  return su_marks_bytes(n) + (one_cta > cluster ? one_cta : cluster);
+  const size_t reg = n > 0 ? su_reg_scratch_bytes(n, max_rows) : 0;
+  const size_t most = one_cta > cluster ? one_cta : cluster;
+  return su_marks_bytes(n) + (most > reg ? most : reg);
 }
 
 extern "C" int dqz_simple_update(const dqz_graph_t *g, void *tensors, double *lambdas, const int32_t *edges,
@@ -812,8 +774,21 @@ extern "C" int dqz_simple_update(const dqz_graph_t *g, void *tensors, double *la
   // one-CTA kernel. Knob DQZ_TUNE_SU_ONCHIP: 1 = the one-CTA kernel only,
   // 2 = the cluster forms at any batch size, 3 = no global-workspace form.
   const int knob = dqz_get_tuning(DQZ_TUNE_SU_ONCHIP);
+  // jobs whose factors fit the registers (bonds up to 16 between degree-3 nodes)
+  // first, whatever the batch size; the forms below take the jobs it left. Measured
+  // at bond 16, ms for a layer of gates: 60 gates (levels of 1 to 11) 3.5 here, 6.7 on
+  // the cluster forms, 20 on the one-CTA kernel; 3,600 gates 16.4, 34.9, 55.9.
+  int chained = 0;
+  if (knob == 0) {
+    marks = static_cast<uint8_t *>(scratch);
+    const int st = su_reg(g, tensors, lambdas, edges, ctrl_is_first, halves, ranks, n, eps, max_rank, max_rows, err,
+                          entropy, marks, job_scratch, su_reg_scratch_bytes(n, max_rows), stream);
+    if (st != DQZ_OK) return st;
+    chained = 1;
+  }
+  const bool larger = !chained || max_rows / 2 > 256 || max_cols > 32;  // a job may be above the register form
   const int pairs = n < sms / 2 ? n : sms / 2;  // one CTA per SM, two per cluster
-  if (max_rows >= SUF_MIN_ROWS && (knob == 4 || (knob == 0 && n > sms))) {
+  if (larger && max_rows >= SUF_MIN_ROWS && (knob == 4 || (knob == 0 && n > sms))) {
     // large batches (and knob 4): every 256-row job on the global-workspace
     // cluster form, 256 threads a CTA, two clusters per SM pair (measured at
     // bond 16: 3,924 jobs in 35.4 ms against 40.2 ms on the one-CTA kernel;
@@ -823,16 +798,16 @@ extern "C" int dqz_simple_update(const dqz_graph_t *g, void *tensors, double *la
     const int cp = su_cluster_pairs(n) < sms ? su_cluster_pairs(n) : sms;
     gws<<<2 * cp, 256, 0, stream>>>(*g, (cd *)tensors, lambdas, edges, ctrl_is_first, (const cd *)halves, ranks, n,
                                     eps, max_rank, err, entropy, su_cluster_cap(max_rows, max_cols), marks,
-                                    job_scratch, 0);
+                                    job_scratch, chained);
     DQZ_CHECK_LAUNCH();
-  } else if (max_rows >= SUF_MIN_ROWS && (n <= sms || knob == 2) && knob != 1) {
+  } else if (larger && max_rows >= SUF_MIN_ROWS && (n <= sms || knob == 2) && knob != 1) {
     auto *onchip = simple_update_onchip_kernel<SUF_THREADS, 1>;
     DQZ_SMEM_ATTR_ONCE(onchip, SUF_SMEM_MAX);
     const long long cap = (long long)(SUF_SMEM_MAX / sizeof(cd));
     marks = static_cast<uint8_t *>(scratch);
     onchip<<<2 * pairs, SUF_THREADS, SUF_SMEM_MAX, stream>>>(
         *g, (cd *)tensors, lambdas, edges, ctrl_is_first, (const cd *)halves, ranks, n, eps, max_rank, err, entropy,
-        cap, marks, nullptr, 0);
+        cap, marks, nullptr, chained);
     DQZ_CHECK_LAUNCH();
     if (knob != 3) {
       const int cp = su_cluster_pairs(n) < pairs ? su_cluster_pairs(n) : pairs;
@@ -907,8 +882,21 @@ extern "C" int dqz_simple_update_noalloc(const dqz_graph_t *g, void *tensors, do
   void *scratch = nullptr;
   const int st = noalloc_address(&scratch);
   if (st != DQZ_OK) return st;
+  // the register form first (as dqz_simple_update), when its marks, one of its
+  // workspace slices and a slice of the kernel below fit the array
+  uint8_t *marks = nullptr;
+  size_t room = (size_t)DQZ_NOALLOC_SCRATCH_BYTES;
+  const size_t mb = su_marks_bytes(n), one = su_reg_scratch_bytes(1, max_rows);
+  if (dqz_get_tuning(DQZ_TUNE_SU_ONCHIP) == 0 && mb + (per_job > one ? per_job : one) <= room) {
+    marks = static_cast<uint8_t *>(scratch);
+    scratch = static_cast<char *>(scratch) + mb;
+    room -= mb;
+    const int rs = su_reg(g, tensors, lambdas, edges, ctrl_is_first, halves, ranks, n, eps, max_rank, max_rows, err,
+                          entropy, marks, scratch, room, stream);
+    if (rs != DQZ_OK) return rs;
+  }
   // as many CTAs as job scratch slices fit in the array; each CTA loops over jobs
-  size_t slots = (size_t)DQZ_NOALLOC_SCRATCH_BYTES / per_job;
+  size_t slots = room / per_job;
   int grid = n < SU_GRID_MAX ? n : SU_GRID_MAX;
   if ((size_t)grid > slots) grid = (int)slots;
   const int tuned = dqz_get_tuning(DQZ_TUNE_SU_GRID);  // the tuned grid, never above the slices
@@ -916,7 +904,7 @@ extern "C" int dqz_simple_update_noalloc(const dqz_graph_t *g, void *tensors, do
   DQZ_SMEM_ATTR_ONCE(simple_update_kernel, SMEM_LIMIT);
   simple_update_kernel<<<grid, GATE_THREADS, smem, stream>>>(*g, (cd *)tensors, lambdas, edges, ctrl_is_first,
                                                              (const cd *)halves, ranks, n, eps, max_rank, max_rows,
-                                                             max_cols, err, entropy, (cd *)scratch, nullptr);
+                                                             max_cols, err, entropy, (cd *)scratch, marks);
   DQZ_CHECK_LAUNCH();
   return DQZ_OK;
 }

@@ -43,25 +43,42 @@ __device__ __forceinline__ void rr_pair(int step, int i, int np, int &p, int &q)
   }
 }
 
-// Unitary J = D R that diagonalises the Hermitian 2x2 [[a, c], [conj(c), b]]
-// (a, b real): D = diag(c/|c|, 1), R the real Jacobi rotation of
-// [[a, |c|], [|c|, b]]. Returns false when c is negligible.
-// One reciprocal square root gives both 1/|c| (phase and tau) and no
-// divisions by |c|; cos = 1/sqrt(1 + t^2) is another (FP64 division and
-// square root are long instruction sequences, and this runs per pair and step).
-__device__ __forceinline__ bool jacobi_rot(double a, double b, cd c, Rot &r) {
+// The rotation that zeroes c in the Hermitian 2x2 [[a, c], [conj(c), b]] (a, b
+// real): J = D R, D = diag(ph, 1) with ph = c / |c|, R = [[cs, sn], [-sn, cs]],
+// t = sn / cs, ac = |c|. False when c is negligible.
+// The tangent is only a direction: a relative error of 1e-7 leaves 1e-7 of c,
+// which the next sweep removes, so it is formed in FP32; cs is then 1 / sqrt(1 +
+// t^2) of that very t, and ph the normalised c, both in FP64, so J is unitary
+// to rounding. This runs per pair and step as one dependent chain.
+struct PhaseRot {
+  cd ph;
+  double cs, sn, t, ac;
+};
+__device__ __forceinline__ bool phase_rot(double a, double b, cd c, PhaseRot &r) {
   const double ac2 = cabs2(c);
-  if (!(ac2 > 1e-300)) return false;
-  const double inv_ac = rsqrt(ac2);
-  const double tau = (b - a) * 0.5 * inv_ac;
-  const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-  const double cs = rsqrt(1.0 + t * t);
-  const double sn = t * cs;
-  const cd ph = mk(c.x * inv_ac, c.y * inv_ac);
-  r.j00 = cscale(ph, cs);
-  r.j01 = cscale(ph, sn);
-  r.j10 = mk(-sn, 0.0);
-  r.j11 = mk(cs, 0.0);
+  if (!(ac2 > 1e-290 && ac2 < 1e290)) return false;
+  const double inv = fast_rsqrt(ac2);
+  const double zeta = (b - a) * 0.5 * inv;
+  const float z = (float)fabs(zeta);
+  // t = 1 / (|zeta| + sqrt(1 + zeta^2)); |zeta| = |b - a| / 2 |c| is below 1e33 for a pair
+  // above the convergence thresholds
+  const float tf = z > 1e8f ? __fdividef(0.5f, z * 1e-8f) * 1e-8f : __fdividef(1.0f, z + __fsqrt_rn(fmaf(z, z, 1.0f)));
+  r.t = zeta >= 0.0 ? (double)tf : -(double)tf;
+  r.cs = fast_rsqrt(fma(r.t, r.t, 1.0));
+  r.sn = r.t * r.cs;
+  r.ph = mk(c.x * inv, c.y * inv);
+  r.ac = ac2 * inv;
+  return true;
+}
+
+// The same as a matrix.
+__device__ __forceinline__ bool jacobi_rot(double a, double b, cd c, Rot &r) {
+  PhaseRot p;
+  if (!phase_rot(a, b, c, p)) return false;
+  r.j00 = cscale(p.ph, p.cs);
+  r.j01 = cscale(p.ph, p.sn);
+  r.j10 = mk(-p.sn, 0.0);
+  r.j11 = mk(p.cs, 0.0);
   return true;
 }
 
@@ -444,6 +461,31 @@ static __device__ void complete_orthonormal(cd *U, int ldu, int m, int ncol, int
   __syncthreads();
 }
 
+// zlarfg's scalars for a column with head alpha and squared norm s below it
+// (not both trivial): beta = -sign(Re alpha) |column|, tau, and the scale 1 /
+// (alpha - beta) of the vector. 1 / beta comes with the norm.
+__device__ __forceinline__ void householder_scalars(cd alpha, double s, double &beta, cd &tau, cd &sc) {
+  const double n2 = cabs2(alpha) + s;
+  double ib;
+  if (fast_range(n2)) {
+    const double inv = fast_rsqrt(n2);
+    beta = -copysign(n2 * inv, alpha.x);
+    ib = -copysign(inv, alpha.x);
+  } else {
+    beta = -copysign(sqrt(n2), alpha.x);
+    ib = 1.0 / beta;
+  }
+  tau = mk((beta - alpha.x) * ib, -alpha.y * ib);
+  const cd den = mk(alpha.x - beta, alpha.y);
+  const double d2 = cabs2(den);
+  if (fast_range(d2)) {
+    const double id = fast_rcp(d2);
+    sc = mk(den.x * id, -den.y * id);
+  } else {
+    sc = cdiv(mk(1.0, 0.0), den);
+  }
+}
+
 // LAPACK-convention Householder QR of A (M x K, column-major, ld = M):
 // H_j = I - tau_j v_j v_j^H, v_j[j] = 1, v_j below the diagonal of column j,
 // R on and above the diagonal, beta real (zlarfg). H_j^H is applied to the
@@ -501,9 +543,9 @@ __device__ __forceinline__ void qr_make_reflector(cd *A, int M, int j, cd *tau) 
   const cd alpha = col[j];
   cd t = czero();
   if (!(s == 0.0 && alpha.y == 0.0)) {
-    const double beta = -copysign(sqrt(cabs2(alpha) + s), alpha.x);
-    t = mk((beta - alpha.x) / beta, -alpha.y / beta);
-    const cd sc = cdiv(mk(1.0, 0.0), mk(alpha.x - beta, alpha.y));
+    double beta;
+    cd sc;
+    householder_scalars(alpha, s, beta, t, sc);
     for (int r = j + 1 + lane; r < M; r += 32) col[r] = cmul(col[r], sc);
     __syncwarp();
     if (lane == 0) col[j] = mk(beta, 0.0);

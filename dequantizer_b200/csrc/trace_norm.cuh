@@ -14,7 +14,7 @@
 // overflow nor underflow.
 #pragma once
 
-#include "common.cuh"
+#include "linalg.cuh"
 
 namespace dqz {
 
@@ -51,12 +51,10 @@ static __device__ double warp_trace_norm(const cd *A, int lda, int n, TraceNormS
       if (xn2 == 0.0 && al.y == 0.0) {
         if (lane == 0) S.e[k] = al.x;
       } else {
-        const double beta = -copysign(sqrt(cabs2(al) + xn2), al.x);
-        const double ib = 1.0 / beta;
-        const cd tau = mk((beta - al.x) * ib, -al.y * ib);
-        const cd den = mk(al.x - beta, al.y);
-        const double id = 1.0 / cabs2(den);
-        const cd v = r == k + 1 ? mk(1.0, 0.0) : (r > k + 1 ? cmul(x, mk(den.x * id, -den.y * id)) : czero());
+        double beta;
+        cd tau, sc;
+        householder_scalars(al, xn2, beta, tau, sc);
+        const cd v = r == k + 1 ? mk(1.0, 0.0) : (r > k + 1 ? cmul(x, sc) : czero());
         if (half == 0) S.v[r] = v;
         if (lane == 0) S.e[k] = beta;
         __syncwarp();
