@@ -504,12 +504,12 @@ class BatchedAnnealer:
             if cols > _lib.MAX_CHI:
                 raise NotImplementedError(f"bond x gate rank {cols} above {_lib.MAX_CHI}")
             n = b1 - b0
-            nb = _lib.lib().dqz_simple_update_scratch_bytes(n, rows, cols)
+            nb = _lib.lib().dqz_simple_update_workspace_bytes(n, rows, cols)
             scratch = torch.empty(nb, dtype=torch.uint8, device=dev)
-            _lib.call("dqz_simple_update", L.gptr, self.G.data_ptr(), self.lam.data_ptr(),
+            _lib.call("dqz_simple_update_ws", L.gptr, self.G.data_ptr(), self.lam.data_ptr(),
                       self.gate_edge_dev[b0:].data_ptr(), self.gate_first_dev[b0:].data_ptr(),
                       self.halves_dev[b0:].data_ptr(), ranks_dev[b0:].data_ptr(), n, EPS, self.max_chi, rows, cols,
-                      err[b0:].data_ptr(), ent[b0:].data_ptr(), scratch.data_ptr(), stream)
+                      err[b0:].data_ptr(), ent[b0:].data_ptr(), scratch.data_ptr(), nb, stream)
             L.edge_chi[self.gate_edge[jobs]] = new
         self._err.append((self._layers, self.level_perm, err, ent))
         self._layers += 1

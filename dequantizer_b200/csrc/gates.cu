@@ -740,20 +740,25 @@ extern "C" size_t dqz_simple_update_scratch_bytes(int32_t n, int32_t max_rows, i
   const size_t cluster = (max_rows >= SUF_MIN_ROWS && n > 0)
                              ? (size_t)2 * su_cluster_pairs(n) * su_cluster_cap(max_rows, max_cols) * sizeof(cd)
                              : 0;
-  const size_t reg = n > 0 ? su_reg_scratch_bytes(n, max_rows) : 0;
-  const size_t most = one_cta > cluster ? one_cta : cluster;
-  return su_marks_bytes(n) + (most > reg ? most : reg);
+  return su_marks_bytes(n) + (one_cta > cluster ? one_cta : cluster);
 }
 
-extern "C" int dqz_simple_update(const dqz_graph_t *g, void *tensors, double *lambdas, const int32_t *edges,
-                                 const uint8_t *ctrl_is_first, const void *halves, const int32_t *ranks, int32_t n,
-                                 double eps, int32_t max_rank, int32_t max_rows, int32_t max_cols, double *err,
-                                 double *entropy, void *scratch, cudaStream_t stream) {
+extern "C" size_t dqz_simple_update_workspace_bytes(int32_t n, int32_t max_rows, int32_t max_cols) {
+  const size_t least = dqz_simple_update_scratch_bytes(n, max_rows, max_cols);
+  const size_t reg = n > 0 ? su_marks_bytes(n) + su_reg_scratch_bytes(n, max_rows) : 0;
+  return least > reg ? least : reg;
+}
+
+extern "C" int dqz_simple_update_ws(const dqz_graph_t *g, void *tensors, double *lambdas, const int32_t *edges,
+                                    const uint8_t *ctrl_is_first, const void *halves, const int32_t *ranks, int32_t n,
+                                    double eps, int32_t max_rank, int32_t max_rows, int32_t max_cols, double *err,
+                                    double *entropy, void *scratch, size_t scratch_bytes, cudaStream_t stream) {
   if (!g || !tensors || !lambdas || !edges || !ctrl_is_first || !halves || !ranks || !err || !entropy || !scratch)
     return DQZ_ERR_ARG;
   if (n < 0 || max_rows <= 0 || max_cols <= 0) return DQZ_ERR_ARG;
   if (max_cols > DQZ_MAX_CHI || (long long)max_rows * max_cols >= (1ll << 31)) return DQZ_ERR_UNSUPPORTED;
   if (n == 0) return DQZ_OK;
+  if (scratch_bytes < dqz_simple_update_scratch_bytes(n, max_rows, max_cols)) return DQZ_ERR_ARG;
   const size_t smem = su_smem_bytes(max_cols);
   if (smem > SMEM_LIMIT) return DQZ_ERR_UNSUPPORTED;
   // jobs of A matrices with 256 rows or more (bond 16 and up between degree-3
@@ -778,11 +783,14 @@ extern "C" int dqz_simple_update(const dqz_graph_t *g, void *tensors, double *la
   // first, whatever the batch size; the forms below take the jobs it left. Measured
   // at bond 16, ms for a layer of gates: 60 gates (levels of 1 to 11) 3.5 here, 6.7 on
   // the cluster forms, 20 on the one-CTA kernel; 3,600 gates 16.4, 34.9, 55.9.
+  // A workspace that holds one job's factors is enough: it sets how many jobs are in
+  // flight; one that does not (small bonds, the least scratch) leaves all to the others.
   int chained = 0;
-  if (knob == 0) {
+  const size_t room = scratch_bytes - su_marks_bytes(n);
+  if (knob == 0 && room >= su_reg_scratch_bytes(1, max_rows)) {
     marks = static_cast<uint8_t *>(scratch);
     const int st = su_reg(g, tensors, lambdas, edges, ctrl_is_first, halves, ranks, n, eps, max_rank, max_rows, err,
-                          entropy, marks, job_scratch, su_reg_scratch_bytes(n, max_rows), stream);
+                          entropy, marks, job_scratch, room, stream);
     if (st != DQZ_OK) return st;
     chained = 1;
   }
@@ -830,6 +838,15 @@ extern "C" int dqz_simple_update(const dqz_graph_t *g, void *tensors, double *la
                                                              max_cols, err, entropy, job_scratch, marks);
   DQZ_CHECK_LAUNCH();
   return DQZ_OK;
+}
+
+extern "C" int dqz_simple_update(const dqz_graph_t *g, void *tensors, double *lambdas, const int32_t *edges,
+                                 const uint8_t *ctrl_is_first, const void *halves, const int32_t *ranks, int32_t n,
+                                 double eps, int32_t max_rank, int32_t max_rows, int32_t max_cols, double *err,
+                                 double *entropy, void *scratch, cudaStream_t stream) {
+  return dqz_simple_update_ws(g, tensors, lambdas, edges, ctrl_is_first, halves, ranks, n, eps, max_rank, max_rows,
+                              max_cols, err, entropy, scratch,
+                              n > 0 ? dqz_simple_update_scratch_bytes(n, max_rows, max_cols) : 0, stream);
 }
 
 // ------------------------------------------- simple update, no allocation
@@ -882,12 +899,14 @@ extern "C" int dqz_simple_update_noalloc(const dqz_graph_t *g, void *tensors, do
   void *scratch = nullptr;
   const int st = noalloc_address(&scratch);
   if (st != DQZ_OK) return st;
-  // the register form first (as dqz_simple_update), when its marks, one of its
-  // workspace slices and a slice of the kernel below fit the array
+  // the register form first where dqz_simple_update takes it (the same singular
+  // vector phases), when its marks, one of its workspace slices and a slice of the
+  // kernel below fit the array
   uint8_t *marks = nullptr;
   size_t room = (size_t)DQZ_NOALLOC_SCRATCH_BYTES;
   const size_t mb = su_marks_bytes(n), one = su_reg_scratch_bytes(1, max_rows);
-  if (dqz_get_tuning(DQZ_TUNE_SU_ONCHIP) == 0 && mb + (per_job > one ? per_job : one) <= room) {
+  if (dqz_get_tuning(DQZ_TUNE_SU_ONCHIP) == 0 && mb + (per_job > one ? per_job : one) <= room &&
+      mb + one <= dqz_simple_update_scratch_bytes(n, max_rows, max_cols)) {
     marks = static_cast<uint8_t *>(scratch);
     scratch = static_cast<char *>(scratch) + mb;
     room -= mb;

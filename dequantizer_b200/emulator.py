@@ -304,11 +304,11 @@ class BPQuantumEmulator:
                 cols = max(op[8] for op in q2)
                 err = torch.empty(n, dtype=torch.float64, device=dev)
                 ent = torch.empty(n, dtype=torch.float64, device=dev)
-                nb = _lib.lib().dqz_simple_update_scratch_bytes(n, rows, cols)
+                nb = _lib.lib().dqz_simple_update_workspace_bytes(n, rows, cols)
                 scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device=dev)
-                _lib.call("dqz_simple_update", L.gptr, self._G.data_ptr(), self._lam.data_ptr(), edges.data_ptr(),
+                _lib.call("dqz_simple_update_ws", L.gptr, self._G.data_ptr(), self._lam.data_ptr(), edges.data_ptr(),
                           first.data_ptr(), halves.data_ptr(), ranks.data_ptr(), n, EPS, self.max_chi, rows, cols,
-                          err.data_ptr(), ent.data_ptr(), scratch.data_ptr(), stream)
+                          err.data_ptr(), ent.data_ptr(), scratch.data_ptr(), nb, stream)
                 self._err_chunks.append(err)
                 self._ent_chunks.append(ent)
                 self._seq_chunks.append(torch.tensor([op[9] for op in q2], dtype=torch.int64, device=dev))

@@ -209,12 +209,12 @@ def apply2_to_vidal_canonical(
     ent = torch.empty(1, dtype=torch.float64, device=dev)
     rows, cols = max(m1, m2), k
     scratch = torch.empty(
-        max(_lib.lib().dqz_simple_update_scratch_bytes(1, rows, cols), 1), dtype=torch.uint8, device=dev
+        max(_lib.lib().dqz_simple_update_workspace_bytes(1, rows, cols), 1), dtype=torch.uint8, device=dev
     )
     run_rank = new_chi if accuracy is None else kk
-    _lib.call("dqz_simple_update", layout.gptr, T.data_ptr(), lam.data_ptr(), e_idx.data_ptr(), ctrl.data_ptr(),
+    _lib.call("dqz_simple_update_ws", layout.gptr, T.data_ptr(), lam.data_ptr(), e_idx.data_ptr(), ctrl.data_ptr(),
               halves.data_ptr(), rk.data_ptr(), 1, eps, int(run_rank), rows, cols, err.data_ptr(), ent.data_ptr(),
-              scratch.data_ptr(), _lib.stream_handle())
+              scratch.data_ptr(), scratch.numel(), _lib.stream_handle())
     ei = layout.edge_index[edge.id]
     layout.edge_chi[ei] = run_rank
     ts = layout.unpack_tensors(T)
