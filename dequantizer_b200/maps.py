@@ -151,20 +151,31 @@ class Topology:
         return self._dev_flat
 
     def device_slice_items(self, layout, device):
-        """The (half-edge, slice) work items of every level for the sliced
-        one-launch sweep (dqz_bp_sweep_sliced), from the layout's current bond
-        dimensions: item_half, item_slice, per-level offsets, the largest level."""
+        """The (half-edge, block of slices) work items of every level for the
+        sliced one-launch sweep (dqz_bp_sweep_sliced), from the layout's current
+        bond dimensions: item_half, item_slice (first slice, plus their number
+        << 16), per-level offsets, the largest level. A block holds up to
+        SLICE_BLOCK_ELEMS entries; in a level of few half-edges, fewer, so that
+        the level's blocks still fill the SMs."""
         key = layout.edge_chi.tobytes()
         cache = self.__dict__.setdefault("_dev_items", {})
         if key not in cache:
             he = layout.half_edge
             ce = np.where(he >= 0, layout.edge_chi[np.maximum(he, 0)], 0).astype(np.int64)
+            size = layout.node_sizes()[layout.half_node] // np.maximum(ce, 1)  # entries of a slice
             halves, slices, off = [], [], [0]
             for lv in self.levels:
-                c = ce[lv]
-                halves.append(np.repeat(lv, c))
-                slices.append(np.concatenate([np.arange(x) for x in c]) if len(c) else np.zeros(0, np.int64))
-                off.append(off[-1] + int(c.sum()))
+                c, sz = ce[lv], size[lv]
+                elems = SLICE_BLOCK_ELEMS
+                while elems > 256 and int(np.ceil(c / np.maximum(elems // np.maximum(sz, 1), 1)).sum()) < SLICE_SMS:
+                    elems //= 2
+                n = np.maximum(elems // np.maximum(sz, 1), 1)
+                cnt = np.where(c > 0, -(-c // n), 0)
+                idx = np.repeat(np.arange(len(lv)), cnt)
+                first = (np.arange(len(idx)) - np.repeat(np.cumsum(cnt) - cnt, cnt)) * n[idx]
+                halves.append(np.asarray(lv)[idx])
+                slices.append(first + (np.minimum(n[idx], c[idx] - first) << 16))
+                off.append(off[-1] + len(idx))
             ih = np.concatenate(halves).astype(np.int32)
             isl = np.concatenate(slices).astype(np.int32)
             widest = int(np.max(np.diff(off))) if len(off) > 1 else 0
@@ -254,6 +265,8 @@ BF16_KERNELS = {"tcgen05": "dqz_bp_node_update_k3_umma", "mma_sync": "dqz_bp_nod
 # half-edges) over the grid: at bond 32 a level of the heavy-hex DFS schedule
 # has a handful of half-edges of ~50 MFLOP each
 SLICED_MIN_CHI = 8
+SLICE_BLOCK_ELEMS = 4096  # entries of a block of slices (bp_slices.cuh)
+SLICE_SMS = 148
 
 
 def bp_sweep(layout: GraphLayout, topo: Topology, T, n2e_old, e2n_old, n2e_new, e2n_new, mid_event=None,

@@ -179,7 +179,9 @@ int dqz_pack_bf16_umma_nodes(const dqz_graph_t *g, const void *tensors_c64, void
  * memory (use the per-level launches then). Small nodes (slices up to 256
  * elements) with narrow levels run in one CTA instead: a warp per half-edge,
  * a CTA barrier between levels, the same results (knob
- * DQZ_TUNE_SWEEP_ONECTA). */
+ * DQZ_TUNE_SWEEP_ONECTA). For bonds below 8 the messages are those of the
+ * per-level launches bit for bit; above, dqz_bp_node_update contracts on the
+ * FP64 tensor cores (as dqz_bp_sweep_sliced does) and agrees to rounding. */
 int dqz_bp_sweep_levels(const dqz_graph_t *g, const void *tensors, const void *n2e_old, const void *e2n_old,
                         void *n2e_new, void *e2n_new, const uint8_t *src_sel, const uint8_t *edge_new,
                         const int32_t *halves, const int32_t *level_off, int32_t n_levels, int32_t max_level,
@@ -203,12 +205,13 @@ int dqz_bp_sweep_planned(const dqz_graph_t *g, const void *tensors, const void *
                          const int32_t *level_off, int32_t n_levels, int32_t max_level, int32_t max_slice,
                          int32_t max_chi, cudaStream_t stream);
 
-/* The same sweep for large bonds: the work items of level l are
- * (item_half[i], item_slice[i]) for i in item_off[l] .. item_off[l+1] (every
- * slice of the bond of every half-edge of the level), spread over the grid;
- * each writes one column of its unnormalised message, then a second barrier
- * pass divides each message of the level by its trace. Bit-identical to the
- * per-level launches; max_items bounds the items of one level. */
+/* The same sweep for bonds from 8: the work items of level l are item_half[i] and
+ * a block of slices of its bond, item_slice[i] = first slice + (number << 16)
+ * (number 0: one), for i in item_off[l] .. item_off[l+1], covering every slice of
+ * every half-edge of the level, spread over the grid. Each writes its columns
+ * of the unnormalised message; readers divide by the trace, and all messages
+ * are divided at the end, before the edge pass. Bit-identical to the per-level
+ * launches; max_items bounds the items of one level. */
 int dqz_bp_sweep_sliced(const dqz_graph_t *g, const void *tensors, const void *n2e_old, const void *e2n_old,
                         void *n2e_new, void *e2n_new, const uint8_t *src_sel, const uint8_t *edge_new,
                         const int32_t *halves, const int32_t *level_off, const int32_t *item_half,
