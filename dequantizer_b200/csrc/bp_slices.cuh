@@ -218,17 +218,11 @@ __device__ __forceinline__ void sl_contract(const SliceItem &it, const cd *buf, 
   }
 }
 
-// Columns a0 .. a0 + n - 1 of the unnormalised outgoing message: put(a', a, value).
-// sl_load has been issued. mx, my: the other bonds' messages; tx, ty: divide them
-// by their traces. Whole CTA; ends with a barrier.
-template <typename Put>
-__device__ __forceinline__ void sl_columns(const SliceItem &it, const cd *mx, bool tx, const cd *my, bool ty, cd *buf,
-                                           cd *sM, Put put) {
+// The other bonds' messages applied to the block. Whole CTA; ends with a barrier
+// (when there is another bond).
+__device__ __forceinline__ void sl_apply(const SliceItem &it, cd *buf, const cd *sM) {
   const SliceGeom &g = it.g;
   const unsigned row = (unsigned)(g.qy * g.d);
-  sl_messages(g, mx, tx, my, ty, sM, sM + 2 * SL_MAX * SL_MS);
-  cp_async_wait<0>();
-  __syncthreads();
   if (g.nb > 0) {
     const FastDiv f(row);
     sl_mode(buf, sM, g.qx, g.sx, it.n * (int)row, row >= 8, [&](int c) {
@@ -244,6 +238,18 @@ __device__ __forceinline__ void sl_columns(const SliceItem &it, const cd *mx, bo
       return (int)(a * (unsigned)g.slice + xx * (unsigned)g.sx + (r - xx * (unsigned)g.d));
     });
   }
+}
+
+// Columns a0 .. a0 + n - 1 of the unnormalised outgoing message: put(a', a, value).
+// sl_load has been issued. mx, my: the other bonds' messages; tx, ty: divide them
+// by their traces. Whole CTA; ends with a barrier.
+template <typename Put>
+__device__ __forceinline__ void sl_columns(const SliceItem &it, const cd *mx, bool tx, const cd *my, bool ty, cd *buf,
+                                           cd *sM, Put put) {
+  sl_messages(it.g, mx, tx, my, ty, sM, sM + 2 * SL_MAX * SL_MS);
+  cp_async_wait<0>();
+  __syncthreads();
+  sl_apply(it, buf, sM);
   int b0 = 0;
   for (; b0 + 4 <= it.n; b0 += 4) sl_contract<4, 2, 4>(it, buf, b0, put);
   if (b0 + 2 <= it.n) {

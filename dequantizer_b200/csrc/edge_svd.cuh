@@ -27,6 +27,11 @@
 
 namespace dqz {
 
+const double F32_MAX = 3.4028234663852886e38;
+
+__device__ __forceinline__ double safe_inverse(double l, double eps) { return 1.0 / ((l < eps ? F32_MAX : 0.0) + l); }
+__device__ __forceinline__ double safe_truncate(double l, double eps) { return l > eps ? l : 0.0; }
+
 constexpr int ES_MAX = 16, ES_LD = 17;
 constexpr unsigned long long ES_MARK = 0x7ff80000000000e5ull;  // in lambda[0]: edge left to the other kernel
 
@@ -218,6 +223,130 @@ __device__ __forceinline__ bool edge_svd_factored(EdgeSmem &S, const cd *mf, con
   const double limit = 0.5 / eps;
   if (!(nf < limit) || !(nb < limit)) return false;
   if (lane < c) lam[lane] = kept;
+  return true;
+}
+
+// Bonds from 17 to 32, one CTA per edge: eigendecompositions of both messages and
+// the SVD, each a one-sided Jacobi iteration of 16 warps' halves or of one half.
+// For a positive semidefinite message m = U S V^H is V S V^H, so its columns'
+// Jacobi gives eigenvalues and eigenvectors; f runs on the first 256 threads, b on
+// the others. In the eigenvector bases C is diag(w_f) V_f^H conj(V_b) diag(w_b),
+// w = sqrt(eigenvalue), = U'' S V''^H, and
+//   G_f = V_f diag(1 / w_f) U'',  G_b = V_b diag(1 / w_b) conj(V''),
+// which takes three products on the FP64 tensor cores instead of seven sums over
+// the bond per entry. Eigenvalues up to eps are dropped as the reference does, so
+// rank-deficient messages (leaves of a graph) are no special case. The Jacobi of a
+// matrix with a negative eigenvalue may mix it with a positive one of the same
+// size: where a column above rounding has no positive U^H V, and for non-finite
+// entries, the edge is marked and left to the kernel with two-sided rotations.
+struct EdgeCtaSmem {
+  static constexpr int LD = RJ_MAX + 1;
+  cd X[2][RJ_MAX * LD], V[2][RJ_MAX * LD];  // column-major: f, b
+  double w[2][RJ_MAX], wi[2][RJ_MAX], s[RJ_MAX];
+  int perm[RJ_MAX];
+  unsigned mask;
+  double scale;
+  JacobiSmem E[2];
+};
+constexpr int EC_THREADS = 2 * RJ_THREADS;
+
+// As edge_svd_factored, for c up to 32 and a whole CTA of EC_THREADS.
+static __device__ bool edge_svd_cta(EdgeCtaSmem &S, const cd *mf, const cd *mb, int c, double eps, cd *Gf, cd *Gb,
+                                    double *lam) {
+  constexpr int LD = EdgeCtaSmem::LD;
+  const int side = threadIdx.x / RJ_THREADS, tid = threadIdx.x % RJ_THREADS, lane = tid & 31, w = threadIdx.x >> 5;
+  const cd *m = side ? mb : mf;
+  cd *X = S.X[side], *V = S.V[side];
+  __syncthreads();  // the previous edge's reads
+  for (int i = tid; i < RJ_MAX * RJ_MAX; i += RJ_THREADS) {
+    const int row = i / RJ_MAX, col = i % RJ_MAX;
+    X[row * LD + col] = row < c && col < c ? m[row * c + col] : czero();
+    V[row * LD + col] = czero();
+  }
+  jacobi_sync(1 + side);
+  cd sym[RJ_MAX * RJ_MAX / RJ_THREADS];  // (m + m^H) / 2
+#pragma unroll
+  for (int j = 0; j < RJ_MAX * RJ_MAX / RJ_THREADS; ++j) {
+    const int i = tid + j * RJ_THREADS, row = i / RJ_MAX, col = i % RJ_MAX;
+    const cd u = X[row * LD + col], l = X[col * LD + row];
+    sym[j] = mk(0.5 * (u.x + l.x), 0.5 * (u.y - l.y));
+  }
+  jacobi_sync(1 + side);
+#pragma unroll
+  for (int j = 0; j < RJ_MAX * RJ_MAX / RJ_THREADS; ++j) {
+    const int i = tid + j * RJ_THREADS;
+    X[(i % RJ_MAX) * LD + i / RJ_MAX] = sym[j];
+  }
+  jacobi_sync(1 + side);
+  cta_jacobi(X, V, LD, c, S.w[side], S.E[side], 1 + side);
+  int bad = 0;
+  if (tid < 32) {
+    const double s = lane < c ? S.w[side][lane] : 0.0;
+    double dot = 0.0;
+    if (lane < c)
+      for (int i = 0; i < c; ++i) {
+        const cd u = X[lane * LD + i], v = V[lane * LD + i];
+        dot += u.x * v.x + u.y * v.y;
+      }
+    double top = s;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    bad = s > 1e-13 * top && !(dot > 0.5);
+    bad |= !(top > 0.0 && top < 1e300);  // zero, or not finite (no column was above the null threshold)
+    const double l = dot < 0.0 ? -s : s;
+    __syncwarp();
+    if (lane < c) {
+      S.w[side][lane] = sqrt(safe_truncate(l, eps));
+      S.wi[side][lane] = sqrt(safe_inverse(l, eps));
+    } else {
+      S.w[side][lane] = S.wi[side][lane] = 0.0;
+    }
+  }
+  if (__syncthreads_or(bad)) return false;
+  // C'' in the first 256 threads' buffer: warps 0-15 take 8 x 8 tiles
+  const int r0 = 8 * (w >> 2), c0 = 8 * (w & 3);
+  CTile<1, 1> t;
+  t.clear();
+  cgemm<true, true, 4>(
+      t, [&](int i, int k) { return S.V[0][(r0 + i) * LD + k]; }, [&](int k, int j) { return S.V[1][(c0 + j) * LD + k]; });
+  ctile_each(t, [&](int i, int j, cd v) { S.X[0][(c0 + j) * LD + r0 + i] = cscale(v, S.w[0][r0 + i] * S.w[1][c0 + j]); });
+  for (int i = threadIdx.x; i < RJ_MAX * LD; i += EC_THREADS) S.X[1][i] = czero();
+  __syncthreads();
+  if (side == 0) cta_jacobi(S.X[0], S.X[1], LD, c, S.s, S.E[0], 1);
+  __syncthreads();
+  if (w == 0) {
+    warp_sort_desc(S.s, c, S.perm);
+    const double sj = lane < c ? S.s[S.perm[lane]] : 0.0;
+    const double l0 = sj / sqrt(warp_sum(sj * sj));
+    const double kept = l0 > eps ? l0 : 0.0;
+    const unsigned mask = __ballot_sync(0xffffffffu, lane < c && kept > eps);
+    if (lane == 0) {
+      S.mask = mask;
+      S.scale = 1.0 / sqrt((double)__popc(mask));
+    }
+    if (lane < c) lam[lane] = kept;
+    else S.perm[lane] = 0;
+  }
+  __syncthreads();
+  // the two products: rows r0 .., columns c0 .. in descending order
+  const unsigned mask = S.mask;
+  const double scale = S.scale;
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    const double *wi = S.wi[f];
+    const cd *Vf = S.V[f], *B = S.X[f];
+    t.clear();
+    const auto la = [&](int i, int k) { return Vf[k * LD + r0 + i]; };
+    const auto lb = [&](int k, int j) { return cscale(B[S.perm[c0 + j] * LD + k], wi[k]); };
+    if (f == 0)
+      cgemm<false, false, 4>(t, la, lb);
+    else
+      cgemm<false, true, 4>(t, la, lb);
+    cd *G = f ? Gb : Gf;
+    ctile_each(t, [&](int i, int j, cd v) {
+      if (r0 + i < c && c0 + j < c) G[(r0 + i) * c + c0 + j] = (mask >> (c0 + j)) & 1u ? cscale(v, scale) : czero();
+    });
+  }
   return true;
 }
 

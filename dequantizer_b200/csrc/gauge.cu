@@ -11,6 +11,7 @@
 //  * symmetric      -- tensor_ops.py:189-199 (canonicalize)
 //  * lambdas->msgs  -- mappings/symmetric_gauge.py:50-61
 //  * density        -- mappings/density_matrix.py:16-37
+#include "bp_slices.cuh"
 #include "edge_svd.cuh"
 #include "linalg.cuh"
 #include "trace_norm.cuh"
@@ -25,10 +26,9 @@ constexpr int WARP_MAX_CHI = 16;     // largest bond of the one-warp kernels
 constexpr int WARP_ROTS = 17;        // rotation slots per warp (n / 2 + 1 for n <= 32)
 constexpr size_t WARP_BLOCK_SMEM = 96 * 1024;
 constexpr int SCRATCH_GRID = 148 * 4;
-const double F32_MAX = 3.4028234663852886e38;
 
-__device__ __forceinline__ double safe_inverse(double l, double eps) { return 1.0 / ((l < eps ? F32_MAX : 0.0) + l); }
-__device__ __forceinline__ double safe_truncate(double l, double eps) { return l > eps ? l : 0.0; }
+// Left to another kernel (edges: in lambda[0]; nodes: in rho[0]).
+__device__ __forceinline__ bool is_marked(double x) { return __double_as_longlong(x) == (long long)ES_MARK; }
 
 // ----------------------------------------------------------- vidal edges
 // Work buffers per edge (each chi^2 complex): Af Vf Ab Vb Qf Qb C W, plus
@@ -52,7 +52,8 @@ __host__ __device__ inline size_t round16(size_t x) { return (x + 15) & ~(size_t
 __global__ void __launch_bounds__(GAUGE_THREADS) vidal_edges_kernel(dqz_graph_t g, const cd *__restrict__ n2e,
                                                                      double eps, cd *orth, double *lambdas,
                                                                      int max_chi, unsigned char *scratch,
-                                                                     const int32_t *__restrict__ sel, int n_sel) {
+                                                                     const int32_t *__restrict__ sel, int n_sel,
+                                                                     int only_marked) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double *red = reinterpret_cast<double *>(smem_raw);
   Rot *rots = reinterpret_cast<Rot *>(smem_raw + 48 * sizeof(double));
@@ -70,6 +71,7 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_edges_kernel(dqz_graph_t 
   const int total = sel ? n_sel : g.n_edges;
   for (int it = blockIdx.x; it < total; it += gridDim.x) {
     const int e = sel ? sel[it] : it;
+    if (only_marked && !is_marked(lambdas[g.edge_lam_off[e]])) continue;
     const int h0 = g.edge_half[2 * e], h1 = g.edge_half[2 * e + 1];
     const int c = g.edge_chi[e];
     const cd *mf = n2e + g.half_msg_off[h0];
@@ -175,6 +177,27 @@ __global__ void __launch_bounds__(32 * ES_WARPS, 4) vidal_edges_factored_kernel(
     if (!done && (threadIdx.x & 31) == 0)
       lam[0] = __longlong_as_double((long long)(fits ? ES_MARK : 0x7ff8000000000000ull));
     __syncwarp();
+  }
+}
+
+// One CTA per edge (WARP_MAX_CHI < max_chi <= RJ_MAX); the few it leaves run the
+// kernel above. Bound by the Jacobi rounds' latency (31 of about 1,200 cycles a
+// sweep, two iterations after another). Measured at 144 edges of bond 32: 768 us,
+// 3,433 us with two-sided rotations and C formed in the original basis.
+__global__ void __launch_bounds__(EC_THREADS) vidal_edges_cta_kernel(dqz_graph_t g, const cd *__restrict__ n2e,
+                                                                     double eps, cd *orth, double *lambdas, int max_chi,
+                                                                     const int32_t *__restrict__ sel, int total) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  EdgeCtaSmem &S = *reinterpret_cast<EdgeCtaSmem *>(smem_raw);
+  for (int it = blockIdx.x; it < total; it += gridDim.x) {
+    const int e = sel ? sel[it] : it;
+    const int c = g.edge_chi[e];
+    double *lam = lambdas + g.edge_lam_off[e];
+    const long long of = g.half_msg_off[g.edge_half[2 * e]], ob = g.half_msg_off[g.edge_half[2 * e + 1]];
+    const bool fits = c <= max_chi;
+    const bool done = fits && edge_svd_cta(S, n2e + of, n2e + ob, c, eps, orth + of, orth + ob, lam);
+    if (!done && threadIdx.x == 0)
+      lam[0] = __longlong_as_double((long long)(fits ? ES_MARK : 0x7ff8000000000000ull));
   }
 }
 
@@ -784,10 +807,131 @@ __global__ void lambdas_to_messages_kernel(dqz_graph_t g, const double *__restri
 }
 
 // -------------------------------------------------------- density matrices
+// Nodes of degree up to 3 with bonds up to 32 whose tensor is above shared memory:
+// block blockIdx.y of the slices of the first bond, one CTA. Slices a' of
+// m_0 T are summed over a from T (read through L2 once per block, whole rows), the
+// other bonds' messages applied in shared memory (bp_slices.cuh), and the block's
+// share of rho summed in a fixed order; density_finish adds the blocks in order.
+// Bound: 1 MB of T per block at bond 32 (16 k cycles of an SM's L2 port).
+// Measured at the 127-qubit heavy-hex lattice, bond 32: 172 us with the finish,
+// 2,049 us with one CTA per node in global scratch.
+constexpr int DENS_BLOCKS = SL_MAX;  // blocks of a node, at most
+constexpr int DENS_PP = DQZ_MAX_PHYS * DQZ_MAX_PHYS;
+constexpr int DENS_GRID = 16;        // blocks in flight per node (the others follow)
+
+__global__ void __launch_bounds__(SL_THREADS, 2) density_slices_kernel(dqz_graph_t g, const cd *__restrict__ Tall,
+                                                                       const cd *__restrict__ e2n,
+                                                                       const int32_t *__restrict__ nodes, cd *rho,
+                                                                       cd *part) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cd *buf = reinterpret_cast<cd *>(smem_raw), *sM = buf + SL_BUF;
+  __shared__ cd sums[SL_THREADS / 32];
+  const int item = blockIdx.x, v = nodes[item], tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  constexpr int NW = SL_THREADS / 32;
+  NodeShape s;
+  load_shape(g, v, s);
+  SliceItem it;
+  if (!sl_geometry(s, 0, it.g)) {
+    if (blockIdx.y == 0 && tid == 0) rho[(long long)item * DENS_PP].x = __longlong_as_double((long long)ES_MARK);
+    return;
+  }
+  const int most = sl_count(it.g), ce = it.g.ce, d = s.d;
+  const unsigned P = (unsigned)it.g.P, row = (unsigned)(it.g.qy * it.g.d);
+  const FastDiv fRow(row);
+  const cd *T = Tall + g.node_off[v], *m0 = e2n + g.half_msg_off[s.half0];
+  const cd *mx = it.g.nb > 0 ? e2n + g.half_msg_off[s.half0 + it.g.fx] : nullptr;
+  const cd *my = it.g.nb > 1 ? e2n + g.half_msg_off[s.half0 + it.g.fy] : nullptr;
+  it.T = T;
+  it.Re = P;
+  for (int blk = blockIdx.y; blk * most < ce; blk += gridDim.y) {
+    it.a0 = blk * most;
+    it.n = ce - it.a0 < most ? ce - it.a0 : most;
+    for (int i = tid; i < it.n * ce; i += SL_THREADS) sM[i] = m0[it.a0 * ce + i];  // rows a0 .. of m_0
+    __syncthreads();
+    for (int b0 = 0; b0 < it.n; b0 += 4) {
+      const int n = it.n - b0;
+      const cd *mr = sM + b0 * ce;
+      for (unsigned x = tid; x < P; x += SL_THREADS) {
+        cd acc[4] = {czero(), czero(), czero(), czero()};
+        if (n >= 3) {
+#pragma unroll 4
+          for (int a = 0; a < ce; ++a) {
+            const cd t = T[(unsigned)a * P + x];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) cfma(acc[j], mr[(j < n ? j : 0) * ce + a], t);
+          }
+        } else {
+#pragma unroll 8
+          for (int a = 0; a < ce; ++a) {
+            const cd t = T[(unsigned)a * P + x];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) cfma(acc[j], mr[(j < n ? j : 0) * ce + a], t);
+          }
+        }
+        const unsigned xx = fRow.div(x);
+        cd *z = buf + b0 * it.g.slice + xx * (unsigned)it.g.sx + (x - xx * row);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < n) z[j * it.g.slice] = acc[j];
+      }
+    }
+    __syncthreads();
+    sl_messages(it.g, mx, false, my, false, sM, sM + 2 * SL_MAX * SL_MS);
+    __syncthreads();
+    sl_apply(it, buf, sM);
+    // rho[si][sj] = sum_b conj(T[b, sj]) Z[b, si]: a group of warps per pair, its warps' sums added in order
+    const int pairs = d * d, group = pairs >= NW ? 1 : NW / pairs, per = NW / group;
+    const unsigned B = (unsigned)it.n * (P / (unsigned)d);
+    const FastDiv fB(P / (unsigned)d);
+    cd *out = part + ((long long)item * DENS_BLOCKS + blk) * DENS_PP;
+    for (int p0 = 0; p0 < pairs; p0 += per) {
+      const int p = p0 + w / group, si = p / d, sj = p % d;
+      cd acc = czero();
+      if (p < pairs && w / group < per)
+#pragma unroll 4
+        for (unsigned b = (w % group) * 32 + lane; b < B; b += 32 * group) {
+          const unsigned a = fB.div(b), r = b - a * (P / (unsigned)d), x = r * (unsigned)d, xx = fRow.div(x);
+          cfmac(acc, T[(unsigned)(it.a0 + a) * P + x + sj],
+                buf[a * (unsigned)it.g.slice + xx * (unsigned)it.g.sx + (x - xx * row) + si]);
+        }
+      acc = warp_csum(acc);
+      if (lane == 0) sums[w] = acc;
+      __syncthreads();
+      if (tid < per && p0 + tid < pairs) {
+        cd t = sums[tid * group];
+        for (int k = 1; k < group; ++k) t = cadd(t, sums[tid * group + k]);
+        out[p0 + tid] = t;
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// rho of the nodes above: the blocks' shares added in order, over the trace.
+__global__ void __launch_bounds__(DENS_PP) density_finish_kernel(dqz_graph_t g, const int32_t *__restrict__ nodes,
+                                                                 cd *rho, const cd *__restrict__ part) {
+  __shared__ cd sh[DENS_PP];
+  const int item = blockIdx.x, v = nodes[item], p = threadIdx.x;
+  NodeShape s;
+  load_shape(g, v, s);
+  SliceGeom geom;
+  if (!sl_geometry(s, 0, geom)) return;
+  const int d = s.d, most = sl_count(geom), blocks = (geom.ce + most - 1) / most;
+  cd t = czero();
+  if (p < d * d)
+    for (int b = 0; b < blocks; ++b) t = cadd(t, part[((long long)item * DENS_BLOCKS + b) * DENS_PP + p]);
+  sh[p] = t;
+  __syncthreads();
+  cd tr = czero();
+  for (int i = 0; i < d; ++i) tr = cadd(tr, sh[i * d + i]);
+  if (p < d * d) rho[(long long)item * DENS_PP + p] = cdiv(t, tr);
+}
+
 __global__ void __launch_bounds__(GAUGE_THREADS) density_kernel(dqz_graph_t g, const cd *__restrict__ Tall,
                                                                  const cd *__restrict__ e2n,
                                                                  const int32_t *__restrict__ nodes, int n_nodes,
-                                                                 cd *rho, int max_size, cd *scratch) {
+                                                                 cd *rho, int max_size, cd *scratch,
+                                                                 int only_marked) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cd *bufA = scratch ? scratch + (long long)blockIdx.x * 2 * max_size : reinterpret_cast<cd *>(smem_raw);
   cd *bufB = bufA + max_size;
@@ -795,6 +939,7 @@ __global__ void __launch_bounds__(GAUGE_THREADS) density_kernel(dqz_graph_t g, c
   __shared__ cd trace_sh;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int item = blockIdx.x; item < n_nodes; item += gridDim.x) {
+    if (only_marked && !is_marked(rho[(long long)item * DQZ_MAX_PHYS * DQZ_MAX_PHYS].x)) continue;
     const int v = nodes[item];
     NodeShape s;
     load_shape(g, v, s);
@@ -876,12 +1021,19 @@ extern "C" int dqz_vidal_edges(const dqz_graph_t *g, const void *n2e, double eps
   size_t need = eigh_smem(max_chi) + vidal_edge_bytes(max_chi);
   const bool use_scratch = need > SMEM_LIMIT;
   if (use_scratch && !scratch) return DQZ_ERR_ARG;
+  const bool cta = max_chi <= RJ_MAX && dqz_get_tuning(DQZ_TUNE_GAUGE_PATH) != 2;
+  if (cta) {
+    DQZ_SMEM_ATTR_ONCE(vidal_edges_cta_kernel, SMEM_LIMIT);
+    vidal_edges_cta_kernel<<<total, EC_THREADS, sizeof(EdgeCtaSmem), stream>>>(*g, (const cd *)n2e, eps, (cd *)orth,
+                                                                              lambdas, max_chi, edges, total);
+    DQZ_CHECK_LAUNCH();
+  }
   size_t smem = use_scratch ? eigh_smem(max_chi) : need;
   DQZ_SMEM_ATTR_ONCE(vidal_edges_kernel, SMEM_LIMIT);
   int grid = use_scratch ? (total < SCRATCH_GRID ? total : SCRATCH_GRID) : total;
   vidal_edges_kernel<<<grid, GAUGE_THREADS, smem, stream>>>(*g, (const cd *)n2e, eps, (cd *)orth, lambdas, max_chi,
                                                            use_scratch ? (unsigned char *)scratch : nullptr, edges,
-                                                           total);
+                                                           total, cta);
   DQZ_CHECK_LAUNCH();
   return DQZ_OK;
 }
@@ -1003,10 +1155,29 @@ extern "C" int dqz_density_matrices(const dqz_graph_t *g, const void *tensors, c
   const bool use_scratch = need > SMEM_LIMIT;
   if (use_scratch && !scratch) return DQZ_ERR_ARG;
   DQZ_SMEM_ATTR_ONCE(density_kernel, SMEM_LIMIT);
-  int grid = use_scratch ? (n_nodes < SCRATCH_GRID ? n_nodes : SCRATCH_GRID) : n_nodes;
-  density_kernel<<<grid, GAUGE_THREADS, use_scratch ? 0 : need, stream>>>(
-      *g, (const cd *)tensors, (const cd *)e2n, nodes, n_nodes, (cd *)rho, max_size,
-      use_scratch ? (cd *)scratch : nullptr);
-  DQZ_CHECK_LAUNCH();
+  if (!use_scratch) {
+    density_kernel<<<n_nodes, GAUGE_THREADS, need, stream>>>(*g, (const cd *)tensors, (const cd *)e2n, nodes, n_nodes,
+                                                            (cd *)rho, max_size, nullptr, 0);
+    DQZ_CHECK_LAUNCH();
+    return DQZ_OK;
+  }
+  // Above shared memory: blocks of slices, then the nodes outside that form one CTA
+  // each. The blocks' shares (a slot of DENS_BLOCKS x DENS_PP per node) take less of
+  // the scratch than the node slices they are followed by. Nodes within shared memory
+  // keep the whole-node form: one launch, and no pass over T per block.
+  static_assert((size_t)DENS_BLOCKS * DENS_PP * sizeof(cd) <= SMEM_LIMIT, "the shares fit a node's scratch");
+  DQZ_SMEM_ATTR_ONCE(density_slices_kernel, SMEM_LIMIT);
+  for (int first = 0; first < n_nodes; first += SCRATCH_GRID) {
+    const int n = n_nodes - first < SCRATCH_GRID ? n_nodes - first : SCRATCH_GRID;
+    cd *out = (cd *)rho + (long long)first * DENS_PP;
+    density_slices_kernel<<<dim3(n, DENS_GRID), SL_THREADS, SL_SMEM, stream>>>(
+        *g, (const cd *)tensors, (const cd *)e2n, nodes + first, out, (cd *)scratch);
+    DQZ_CHECK_LAUNCH();
+    density_finish_kernel<<<n, DENS_PP, 0, stream>>>(*g, nodes + first, out, (const cd *)scratch);
+    DQZ_CHECK_LAUNCH();
+    density_kernel<<<n, GAUGE_THREADS, 0, stream>>>(*g, (const cd *)tensors, (const cd *)e2n, nodes + first, n, out,
+                                                    max_size, (cd *)scratch, 1);
+    DQZ_CHECK_LAUNCH();
+  }
   return DQZ_OK;
 }

@@ -262,8 +262,29 @@ __device__ __forceinline__ void cta_jacobi_v(cd *V, int ld, int n, int p, int q,
   }
 }
 
-static __device__ void cta_jacobi(cd *X, cd *V, int ld, int n, double *s, JacobiSmem &E) {
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+// Barrier of this Jacobi's RJ_THREADS threads: the CTA's (id 0), or a named one
+// where a CTA runs two at once (its warps 8 .. 15 the second).
+__device__ __forceinline__ void jacobi_sync(int bar) {
+  if (bar == 0)
+    __syncthreads();
+  else
+    asm volatile("bar.sync %0, 256;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ int jacobi_any(int bar, int v) {
+  if (bar == 0) return __syncthreads_or(v);
+  int r;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n bar.red.or.pred q, %2, 256, p;\n selp.s32 %0, 1, 0, q;\n}"
+      : "=r"(r)
+      : "r"(v), "r"(bar)
+      : "memory");
+  return r;
+}
+
+// Called by all RJ_THREADS threads of the barrier `bar`.
+static __device__ void cta_jacobi(cd *X, cd *V, int ld, int n, double *s, JacobiSmem &E, int bar = 0) {
+  static_assert(RJ_THREADS == 256, "the named barrier's threads");
+  const int tid = threadIdx.x % RJ_THREADS, lane = tid & 31, w = tid >> 5;
   const int grp = (tid & 127) >> 3, sub = tid & 7;
   const int np = n + (n & 1), npairs = np / 2;
   const bool main = tid < 128, seat = grp < npairs;
@@ -275,7 +296,7 @@ static __device__ void cta_jacobi(cd *X, cd *V, int ld, int n, double *s, Jacobi
     f = warp_sum(f);
     if (lane == 0) E.fro[w] = f;
   }
-  __syncthreads();
+  jacobi_sync(bar);
   const double null_thr = hestenes_null_scale(n) * (((E.fro[0] + E.fro[1]) + E.fro[2]) + E.fro[3]);
   int done = 0;  // rounds of all sweeps so far, for the parity of the rotations
   int pp = 0, pq = n;  // V's pair: the round before
@@ -326,9 +347,9 @@ static __device__ void cta_jacobi(cd *X, cd *V, int ld, int n, double *s, Jacobi
         pp = p;
         pq = q;
       }
-      __syncthreads();
+      jacobi_sync(bar);
     }
-    if (!__syncthreads_or(more)) break;
+    if (!jacobi_any(bar, more)) break;
   }
   if (!main && done > 0 && seat && pq < n) cta_jacobi_v(V, ld, n, pp, pq, sub, E, (done - 1) & 1, grp);
   if (main)
@@ -347,7 +368,7 @@ static __device__ void cta_jacobi(cd *X, cd *V, int ld, int n, double *s, Jacobi
         if (in && sub + 8 * i < n) col[8 * i] = cscale(col[8 * i], inv);
       if (in && sub == 0) s[j] = sj;
     }
-  __syncthreads();
+  jacobi_sync(bar);
 }
 
 }  // namespace dqz
