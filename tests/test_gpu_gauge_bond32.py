@@ -85,3 +85,55 @@ def test_density(graph, n, dims, phys):
             y = torch.movedim(torch.tensordot(L.message_view(e2n, h0 + f), y, dims=([1], [f])), 0, f)
         r = torch.einsum("bi,bj->ij", y.reshape(-1, phys), ts[v].conj().reshape(-1, phys))
         assert float((rho[j] - r / r.diagonal().sum()).abs().max()) < 1e-11
+
+
+@pytest.mark.parametrize("dims,phys", [((17,), 2), ((32, 1, 30), 3), ((32,), 2), ((31, 2, 33), 2)])
+def test_distance_terms(dims, phys):
+    """Each half-edge's trace norm (33: the form above bond 32). R sums at most 3 *
+    32^2 products a split, 768 eps = 1.7e-13 of a trace of 1, its trace norm moves
+    by at most 32^(1/2) times the Frobenius norm of that: 1e-12."""
+    L = layout_of(rr3(8, dims, phys))
+    rng = np.random.default_rng(4)
+    T = torch.from_numpy(rng.standard_normal(L.tensor_elems) + 1j * rng.standard_normal(L.tensor_elems)).cuda()
+    lam_h = np.concatenate([np.sort(10.0 ** -rng.uniform(0, 4, int(c)))[::-1] for c in L.edge_chi])
+    lam = torch.from_numpy(lam_h).cuda()
+    part = M.vidal_distance_partial(L, T, lam, 1e-10).cpu().numpy()
+    for v, t in enumerate(L.unpack_tensors(T)):
+        h0 = int(L.node_half[v])
+        ls = [L.lambda_view(lam, int(L.half_edge[h0 + f])) for f in range(3)]
+        for f in range(3):
+            y = t
+            for f2 in range(3):
+                if f2 != f:
+                    y = y * ls[f2].reshape([-1 if i == f2 else 1 for i in range(4)])
+            y = torch.movedim(y, f, 0).reshape(t.shape[f], -1).cpu().numpy()
+            r = y.conj() @ y.T
+            r = r / np.trace(r)
+            on = r.diagonal().real > 1e-10
+            ref = np.abs(np.linalg.eigvalsh(r - np.diag(on / on.sum()))).sum()
+            assert abs(part[h0 + f] - ref) < 1e-12
+
+
+def test_distance_of_diagonal_zero_and_non_finite_tensors():
+    """Graded and diagonal reduced matrices (no reflector, tiny off-diagonals), a zero and a NaN tensor."""
+    L = layout_of(rr3(8, (32,)))
+    T = torch.zeros(L.tensor_elems, dtype=torch.complex128, device="cuda")
+    for v, t in enumerate(L.unpack_tensors(T)):
+        base = int(L.node_off[v])
+        i = torch.arange(32, device="cuda")
+        idx = ((i * 32 + i) * 32 + i) * 2
+        T[base + idx] = (10.0 ** (-0.5 * i)).to(torch.complex128)
+    T[int(L.node_off[5]):int(L.node_off[5]) + 65536] = 0.0
+    T[int(L.node_off[6]) + 7] = complex("nan")
+    lam = torch.ones(L.lam_elems, dtype=torch.float64, device="cuda")
+    part = M.vidal_distance_partial(L, T, lam, 1e-10).cpu().numpy()
+    w = ((10.0 ** (-0.5 * i)).to(torch.complex128).abs() ** 2).cpu().numpy()  # of the entries as stored
+    w /= w.sum()
+    on = w > 1e-10
+    ref = np.abs(w - on / on.sum()).sum()
+    for v in range(8):
+        h0 = int(L.node_half[v])
+        if v in (5, 6):
+            assert not np.isfinite(part[h0:h0 + 3]).any()
+        else:
+            assert np.abs(part[h0:h0 + 3] - ref).max() < 1e-13
