@@ -417,6 +417,249 @@ __device__ __forceinline__ void warp_plan_item(const long long *pw, const cd *__
   __syncwarp();
 }
 
+// ---- the same with all slices of an item at once: the mode products run on the
+// whole tensor (the outgoing bond is one more batch index), so an item is degree -
+// 1 dependent phases instead of that many per slice, and a lane has several outputs
+// of a phase in flight. Every entry is the same sum in the same order. What does not
+// depend on other items of the sweep happens before the barrier that opens
+// its level: the warps take the items of all levels in turn, so that a warp has
+// several levels' time to stage its next item (words, strides and reciprocals, the
+// addresses of its messages, its tensor by cp.async). A quotient x / y is
+// floor((2 x + 1) ceil(2^31 / y) / 2^32): (x + 1/2) / y plus less than (x + 1/2)
+// 2^-31, and (x + 1/2) / y lies at least 1 / (2 y) below a whole number, so it is
+// exact while x y < 2^30.
+// Bound by the levels' chain, and within a level by the SM's shared-memory port (five
+// items' operand loads at once). 16 warps: with 32 the registers spill. Measured on the
+// 6 x 6 x 6 lattice, bond 2 (206 levels, 5 half-edges each): 661 us, 1,750 us by slices.
+struct PlanWarp {
+  long long pw[DQZ_PLAN_WORDS + 1];
+  int4 bond[DQZ_MAX_DEGREE];    // stride R, dimension q, small_div's factors of R and q
+  int moff[DQZ_MAX_DEGREE];     // the bond's message in Ms
+  int size, nm;                 // entries of the tensor and of all messages
+};
+__device__ __forceinline__ unsigned small_div(unsigned x, unsigned m) { return __umulhi(2 * x + 1, m); }
+__device__ __forceinline__ unsigned small_div_factor(unsigned y) { return (0x80000000u + y - 1) / y; }
+
+// The words of the next item, `word` in lane < DQZ_PLAN_WORDS, and what follows from them.
+__device__ __forceinline__ void plan_setup(PlanWarp &W, long long word) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  if (lane < DQZ_PLAN_WORDS) W.pw[lane] = word;
+  __syncwarp();
+  const int k = (int)W.pw[1], e = (int)W.pw[3];
+  const long long *dims = W.pw + 5;
+  if (lane < k) {
+    int R = (int)W.pw[2], off = 0;
+    for (int f = k - 1; f > lane; --f) R *= (int)dims[f];
+    for (int f = 0; f < lane; ++f)
+      if (f != e) off += (int)(dims[f] * dims[f]);
+    const int q = (int)dims[lane];
+    W.bond[lane] = make_int4(R, q, (int)small_div_factor((unsigned)R), (int)small_div_factor((unsigned)q));
+    W.moff[lane] = off;
+    if (lane == 0) W.size = R * q;
+    if (lane == k - 1) W.nm = off + (lane != e ? q * q : 0);
+  }
+  __syncwarp();
+}
+// Address of entry x of the item's messages, laid one after another.
+__device__ __forceinline__ const cd *plan_message(const PlanWarp &W, int x, const cd *n2e_old, const cd *e2n_old,
+                                                  const cd *n2e_new) {
+  const int k = (int)W.pw[1], e = (int)W.pw[3];
+  int slot = 0, at = x;
+  for (int f = 0; f < k; ++f) {
+    if (f == e) continue;
+    if (x >= W.moff[f]) {
+      at = x - W.moff[f];
+      slot = f < e ? f : f - 1;
+    }
+  }
+  const long long code = W.pw[5 + DQZ_MAX_DEGREE + slot];
+  const int src = (int)(code & 3);
+  return (src == DQZ_SRC_E2N_OLD ? e2n_old : (src == DQZ_SRC_N2E_NEW ? n2e_new : n2e_old)) + (code >> 2) + at;
+}
+__device__ __forceinline__ void plan_load_tensor(const PlanWarp &W, const cd *__restrict__ T, cd *Ts) {
+  const cd *Tv = T + W.pw[0];
+  for (int x = threadIdx.x & 31; x < W.size; x += 32) cp_async16(Ts + x, Tv + x);
+  cp_async_commit();
+}
+
+// Y = X x_f m over the whole tensor.
+template <int U>
+__device__ __forceinline__ void plan_product(const int4 &bond, unsigned size, const cd *X, cd *Y, const cd *m) {
+  const unsigned R = (unsigned)bond.x, q = (unsigned)bond.y, fR = (unsigned)bond.z, fq = (unsigned)bond.w;
+  for (unsigned o0 = threadIdx.x & 31; o0 < size; o0 += 32 * U) {
+    cd acc[U];
+    unsigned x[U], mi[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned o = o0 + 32 * u < size ? o0 + 32 * u : o0;
+      const unsigned t = small_div(o, fR), l = small_div(t, fq), i = t - l * q;
+      mi[u] = i * q;
+      x[u] = o - i * R;
+      acc[u] = czero();
+    }
+#pragma unroll 2
+    for (unsigned b = 0; b < q; ++b)
+#pragma unroll
+      for (int u = 0; u < U; ++u) cfma(acc[u], m[mi[u] + b], X[x[u] + b * R]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (o0 + 32 * u < size) Y[o0 + 32 * u] = acc[u];
+  }
+}
+
+// warp_csum of four values, each lane exchanging only what it will go on with: value
+// u's sum, added in the same pairs, ends in lane 8 u.
+__device__ __forceinline__ cd warp_csum4(const cd (&v)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool hi = lane & 16, mid = lane & 8;
+  const auto get = [](cd x, int o) {
+    return mk(__shfl_xor_sync(0xffffffffu, x.x, o), __shfl_xor_sync(0xffffffffu, x.y, o));
+  };
+  const cd a = cadd(hi ? v[2] : v[0], get(hi ? v[0] : v[2], 16));
+  const cd b = cadd(hi ? v[3] : v[1], get(hi ? v[1] : v[3], 16));
+  cd s = cadd(mid ? b : a, get(mid ? a : b, 8));
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s = cadd(s, get(s, o));
+  return s;
+}
+
+// out[p], p = a' ce + a, for four pairs from p0 (up to ce^2): lane-strided sums over x as node_update_half.
+__device__ __forceinline__ void plan_pairs(const int4 &bond, unsigned P, const cd *Ts, const cd *Z, int p0,
+                                           cd *out) {
+  const int lane = threadIdx.x & 31;
+  const unsigned Re = (unsigned)bond.x, ce = (unsigned)bond.y, fR = (unsigned)bond.z;
+  cd acc[4];
+  unsigned tp[4], zp[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const unsigned p = p0 + u < ce * ce ? p0 + u : p0, ap = small_div(p, (unsigned)bond.w);
+    tp[u] = ap * Re;
+    zp[u] = (p - ap * ce) * Re;
+    acc[u] = czero();
+  }
+#pragma unroll 2
+  for (unsigned x = lane; x < P; x += 32) {
+    const unsigned l = small_div(x, fR), base = x + l * (ce - 1) * Re;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) cfmac(acc[u], Ts[base + tp[u]], Z[base + zp[u]]);
+  }
+  const cd s = warp_csum4(acc);
+  const unsigned p = p0 + (lane >> 3);
+  if ((lane & 7) == 0 && p < ce * ce) out[p] = s;
+}
+
+__host__ __device__ inline size_t plan_warp_elems(int max_slice, int max_chi) {
+  return (size_t)max_chi * max_chi + 3 * (size_t)max_slice * max_chi +
+         (size_t)(DQZ_MAX_DEGREE - 1) * max_chi * max_chi;
+}
+__host__ __device__ inline size_t plan_warp_bytes(int max_slice, int max_chi) {
+  return plan_warp_elems(max_slice, max_chi) * sizeof(cd) + round_up16(sizeof(PlanWarp));
+}
+constexpr int PLAN_LEVELS = 1024;  // level offsets kept in shared memory
+constexpr int PLAN_THREADS = 512;
+
+// The edge pass of the one-CTA sweeps, a lane per half-edge: the table look-ups of 32
+// of them in flight at once.
+__device__ __forceinline__ void plan_edge_pass(const dqz_graph_t &g, const cd *n2e_old, const cd *n2e_new, cd *e2n_new,
+                                               const uint8_t *__restrict__ edge_new) {
+  for (int h = threadIdx.x; h < g.n_halves; h += blockDim.x) {
+    const int e = g.half_edge[h];
+    const int tw = g.half_twin[h];
+    if (e < 0 || tw < 0) continue;
+    const int c = g.edge_chi[e];
+    const cd *src = (edge_new[h] ? n2e_new : n2e_old) + g.half_msg_off[tw];
+    cd *dst = e2n_new + g.half_msg_off[h];
+#pragma unroll 4
+    for (int i = 0; i < c * c; ++i) dst[i] = src[i];
+  }
+}
+
+__global__ void __launch_bounds__(PLAN_THREADS) bp_sweep_whole_kernel(
+    dqz_graph_t g, const cd *__restrict__ T, const cd *n2e_old, const cd *e2n_old, cd *n2e_new, cd *e2n_new,
+    const uint8_t *__restrict__ edge_new, const long long *__restrict__ plan, const int32_t *__restrict__ level_off,
+    int n_levels, int max_slice, int max_chi) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int off_sh[PLAN_LEVELS + 1];
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
+  unsigned char *mine = smem_raw + (size_t)warp * plan_warp_bytes(max_slice, max_chi);
+  PlanWarp &W = *reinterpret_cast<PlanWarp *>(mine);
+  cd *out = reinterpret_cast<cd *>(mine + round_up16(sizeof(PlanWarp)));
+  cd *Ts = out + (size_t)max_chi * max_chi, *A = Ts + (size_t)max_slice * max_chi,
+     *B = A + (size_t)max_slice * max_chi, *Ms = B + (size_t)max_slice * max_chi;
+  for (int i = threadIdx.x; i <= n_levels && i <= PLAN_LEVELS; i += blockDim.x) off_sh[i] = level_off[i];
+  __syncthreads();
+  auto offset = [&](int lv) { return lv <= PLAN_LEVELS ? off_sh[lv] : level_off[lv]; };
+  const int total = offset(n_levels);
+  int at = warp;  // the staged item: the warps take the items of all levels in turn
+  long long later = 0;
+  bool pending = false;
+  const cd *mp[2] = {nullptr, nullptr};
+  auto stage = [&](long long word) {  // the item's words, message addresses and tensor
+    plan_setup(W, word);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (lane + 32 * j < W.nm) mp[j] = plan_message(W, lane + 32 * j, n2e_old, e2n_old, n2e_new);
+    plan_load_tensor(W, T, Ts);
+  };
+  auto words = [&](int item) {
+    return item < total && lane < DQZ_PLAN_WORDS ? plan[(long long)item * DQZ_PLAN_WORDS + lane] : 0;
+  };
+  if (at < total) stage(words(at));
+  for (int lv = 0; lv < n_levels; ++lv) {
+    for (const int end = offset(lv + 1); at < end; at += nw) {
+      const long long word = words(at + nw);
+      const int k = (int)W.pw[1], e = (int)W.pw[3], nm = W.nm;
+      const long long *dims = W.pw + 5;
+      const int ce = (int)dims[e];
+      const long long dst_off = W.pw[4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (lane + 32 * j < nm) Ms[lane + 32 * j] = *mp[j];
+      for (int x = lane + 64; x < nm; x += 32) Ms[x] = *plan_message(W, x, n2e_old, e2n_old, n2e_new);
+      cp_async_wait<0>();
+      __syncwarp();
+      const cd *cur = Ts;
+      cd *nxt = A;
+      const unsigned size = (unsigned)W.size;
+      int4 bond = W.bond[e == 0 ? (k > 1 ? 1 : 0) : 0];
+      for (int f = e == 0 ? 1 : 0; f < k;) {
+        const int after = f + 1 == e ? f + 2 : f + 1;
+        const int4 nb = W.bond[after < k ? after : e];  // on its way during the product; the pairs' at the end
+        plan_product<4>(bond, size, cur, nxt, Ms + W.moff[f]);
+        bond = nb;
+        f = after;
+        __syncwarp();
+        cur = nxt;
+        nxt = nxt == A ? B : A;
+      }
+      const unsigned P = size / (unsigned)ce;
+      for (int p0 = 0; p0 < ce * ce; p0 += 4) plan_pairs(bond, P, Ts, cur, p0, out);
+      __syncwarp();
+      cd tr = czero();
+      for (int i = 0; i < ce; ++i) tr = cadd(tr, out[i * ce + i]);
+      cd *dst = n2e_new + dst_off;
+      for (int i = lane; i < ce * ce; i += 32) dst[i] = cdiv(out[i], tr);
+      if (at + nw < total) {
+        // after the barrier, which the other warps wait at, unless it is for this level
+        if (at + nw < end) {
+          stage(word);
+        } else {
+          later = word;
+          pending = true;
+        }
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    if (pending) {
+      stage(later);
+      pending = false;
+    }
+  }
+  plan_edge_pass(g, n2e_old, n2e_new, e2n_new, edge_new);
+}
+
 __global__ void __launch_bounds__(ONECTA_THREADS) bp_sweep_planned_kernel(
     dqz_graph_t g, const cd *__restrict__ T, const cd *n2e_old, const cd *e2n_old, cd *n2e_new, cd *e2n_new,
     const uint8_t *__restrict__ edge_new, const long long *__restrict__ plan, const int32_t *__restrict__ level_off,
@@ -438,15 +681,7 @@ __global__ void __launch_bounds__(ONECTA_THREADS) bp_sweep_planned_kernel(
     }
     __syncthreads();
   }
-  for (int h = warp; h < g.n_halves; h += nw) {
-    const int e = g.half_edge[h];
-    const int tw = g.half_twin[h];
-    if (e < 0 || tw < 0) continue;
-    const int c = g.edge_chi[e];
-    const cd *src = (edge_new[h] ? n2e_new : n2e_old) + g.half_msg_off[tw];
-    cd *dst = e2n_new + g.half_msg_off[h];
-    warp_copy16(reinterpret_cast<uint4 *>(dst), reinterpret_cast<const uint4 *>(src), c * c);
-  }
+  plan_edge_pass(g, n2e_old, n2e_new, e2n_new, edge_new);
 }
 
 // Grid-wide barrier for a cooperative launch: one arrival counter and one
@@ -888,12 +1123,24 @@ extern "C" int dqz_bp_sweep_planned(const dqz_graph_t *g, const void *tensors, c
   while (warps > 8 && round_up16((size_t)warps * DQZ_PLAN_WORDS * sizeof(long long)) + warps * per_warp >
                           BP_SMEM_LIMIT)
     --warps;
-  const size_t smem = round_up16((size_t)warps * DQZ_PLAN_WORDS * sizeof(long long)) + warps * per_warp;
+  size_t smem = round_up16((size_t)warps * DQZ_PLAN_WORDS * sizeof(long long)) + warps * per_warp;
   if (smem > BP_SMEM_LIMIT) return DQZ_ERR_UNSUPPORTED;
-  DQZ_SMEM_ATTR_ONCE(bp_sweep_planned_kernel, BP_SMEM_LIMIT);
-  bp_sweep_planned_kernel<<<1, 32 * warps, smem, stream>>>(
-      *g, (const cd *)tensors, (const cd *)n2e_old, (const cd *)e2n_old, (cd *)n2e_new, (cd *)e2n_new, edge_new,
-      (const long long *)plan, level_off, (int)n_levels, (int)max_slice, (int)max_chi);
+  // all slices of an item at once where the tensors' buffers leave as many warps as a
+  // level can use, or as the form by slices has
+  const size_t per_whole = plan_warp_bytes(max_slice, max_chi);
+  int fit = (int)(BP_SMEM_LIMIT / per_whole);
+  if (fit > PLAN_THREADS / 32) fit = PLAN_THREADS / 32;
+  if (fit >= 1 && (fit >= PLAN_THREADS / 32 || fit >= warps || fit >= max_level)) {
+    DQZ_SMEM_ATTR_ONCE(bp_sweep_whole_kernel, BP_SMEM_LIMIT);
+    bp_sweep_whole_kernel<<<1, 32 * fit, fit * per_whole, stream>>>(
+        *g, (const cd *)tensors, (const cd *)n2e_old, (const cd *)e2n_old, (cd *)n2e_new, (cd *)e2n_new, edge_new,
+        (const long long *)plan, level_off, (int)n_levels, (int)max_slice, (int)max_chi);
+  } else {
+    DQZ_SMEM_ATTR_ONCE(bp_sweep_planned_kernel, BP_SMEM_LIMIT);
+    bp_sweep_planned_kernel<<<1, 32 * warps, smem, stream>>>(
+        *g, (const cd *)tensors, (const cd *)n2e_old, (const cd *)e2n_old, (cd *)n2e_new, (cd *)e2n_new, edge_new,
+        (const long long *)plan, level_off, (int)n_levels, (int)max_slice, (int)max_chi);
+  }
   DQZ_CHECK_LAUNCH();
   return DQZ_OK;
 }
