@@ -16,7 +16,7 @@ and one simple-update launch.
 
 import logging
 import math
-from typing import Dict, List, Optional
+from typing import Dict, List, NamedTuple, Optional
 
 import numpy as np
 import torch
@@ -32,6 +32,11 @@ from .tensor_graph_ops import simple_update_shapes
 log = logging.getLogger(__name__)
 
 EPS = 1e-10  # bp_quantum_emulator.py:84-86, 161
+
+
+class SplitGate(NamedTuple):
+    halves: np.ndarray
+    rank: int
 
 
 class BPQuantumEmulator:
@@ -98,6 +103,9 @@ class BPQuantumEmulator:
     def _grow(self, node_need: Dict[int, int], edge_need: Dict[int, int]):
         """Moves the state into a layout whose capacities cover the given needs."""
         L = self._layout
+        if all(s <= L.node_capacity[v] for v, s in node_need.items()) and all(
+                c <= L.edge_capacity[e] for e, c in edge_need.items()):
+            return
         ncap = L.node_capacity.copy()
         ecap = L.edge_capacity.copy()
         for v, s in node_need.items():
@@ -106,8 +114,6 @@ class BPQuantumEmulator:
         for e, c in edge_need.items():
             if c > ecap[e]:
                 ecap[e] = max(c, 2 * ecap[e])
-        if np.array_equal(ncap, L.node_capacity) and np.array_equal(ecap, L.edge_capacity):
-            return
         full = self._full_capacities()
         if full is not None:  # take the final capacities at once: one arena move instead of one per growing gate
             ncap = np.maximum(ncap, full[0])
@@ -177,14 +183,21 @@ class BPQuantumEmulator:
         self._passed = 0
 
     def apply_q2(self, gate, controlling_node_id, controlled_node_id):
-        """bp_quantum_emulator.py:144-167 (queued; see module docstring)."""
+        """bp_quantum_emulator.py:144-167 (queued; see module docstring). ``gate``
+        may also be a gate's ``split_q2``, for one that is applied many times."""
         if self._passed >= self.per_regauging:
             self._vidal_regauging()
             self._passed = 0
+        halves, rank = gate if isinstance(gate, SplitGate) else self.split_q2(gate)
+        self._queue_q2(controlling_node_id, controlled_node_id, halves, rank)
+        self._passed += 1
+
+    @staticmethod
+    def split_q2(gate) -> "SplitGate":
+        """The two halves of a two-site gate and its rank (tensor_ops.py:202-218)."""
         g = gate.detach().cpu().numpy() if isinstance(gate, torch.Tensor) else np.asarray(gate)
         flat, ranks, _ = decompose_gates(g[None], EPS)
-        self._queue_q2(controlling_node_id, controlled_node_id, flat[0], int(ranks[0]))
-        self._passed += 1
+        return SplitGate(flat[0], int(ranks[0]))
 
     def apply_q1(self, gate, node_id):
         """bp_quantum_emulator.py:175-180 (queued)."""
@@ -232,7 +245,7 @@ class BPQuantumEmulator:
         d = int(self._layout.phys[v])
         if tuple(gate.shape) != (d, d):
             raise ValueError(f"gate of shape {tuple(gate.shape)} does not act on a physical dimension {d}")
-        self._pending.append(("q1", v, gate.reshape(-1)))
+        self._pending.append(("q1", v, gate.detach().cpu().resolve_conj().resolve_neg().reshape(-1).numpy()))
         self._rho_cache = None
 
     def _queue_q2(self, id1, id2, halves: np.ndarray, rank: int):
@@ -252,8 +265,8 @@ class BPQuantumEmulator:
                                                      self.max_chi)
         if k > _lib.MAX_CHI:
             raise NotImplementedError(f"bond dimension x gate rank = {k} above {_lib.MAX_CHI} is not supported")
-        s1 = int(np.prod(d1)) * int(L.phys[v1]) // d1[i1] * new_chi
-        s2 = int(np.prod(d2)) * int(L.phys[v2]) // d2[i2] * new_chi
+        s1 = math.prod(d1) * int(L.phys[v1]) // d1[i1] * new_chi
+        s2 = math.prod(d2) * int(L.phys[v2]) // d2[i2] * new_chi
         self._grow({v1: s1, v2: s2}, {e: new_chi})
         L = self._layout
         first = 1 if edge.neighbors[0] is n1 else 0
@@ -282,36 +295,52 @@ class BPQuantumEmulator:
         self._pending = []
         stream = _lib.stream_handle()
         mp2 = _lib.MAX_PHYS * _lib.MAX_PHYS
+        # the tables of all levels in one buffer and one copy
+        pieces, used = [], 0
+
+        def put(a: np.ndarray) -> int:
+            nonlocal used
+            at = used
+            pieces.append((at, a))
+            used += (a.nbytes + 15) & ~15
+            return at
+
+        runs = []
         for lv in sorted(levels):
-            ops = levels[lv]
-            q1 = [op for op in ops if op[0] == "q1"]
-            q2 = [op for op in ops if op[0] == "q2"]
+            q1 = [op for op in levels[lv] if op[0] == "q1"]
+            q2 = [op for op in levels[lv] if op[0] == "q2"]
             if q1:
-                nodes = torch.tensor([op[1] for op in q1], dtype=torch.int32)
-                gates = torch.zeros((len(q1), mp2), dtype=torch.complex128)
+                gates = np.zeros((len(q1), mp2), dtype=np.complex128)
                 for j, op in enumerate(q1):
-                    gates[j, : op[2].numel()] = op[2].cpu()
-                nodes, gates = nodes.to(dev), gates.to(dev)
-                _lib.call("dqz_apply1", L.gptr, self._G.data_ptr(), nodes.data_ptr(), gates.data_ptr(), len(q1),
-                          stream)
+                    gates[j, : len(op[2])] = op[2]
+                runs.append((len(q1), put(np.array([op[1] for op in q1], dtype=np.int32)), put(gates)))
             if q2:
-                n = len(q2)
-                edges = torch.tensor([op[3] for op in q2], dtype=torch.int32).to(dev)
-                first = torch.tensor([op[4] for op in q2], dtype=torch.uint8).to(dev)
-                halves = torch.from_numpy(np.stack([op[5] for op in q2]).reshape(n, -1)).to(dev)
-                ranks = torch.tensor([op[6] for op in q2], dtype=torch.int32).to(dev)
-                rows = max(op[7] for op in q2)
-                cols = max(op[8] for op in q2)
-                err = torch.empty(n, dtype=torch.float64, device=dev)
-                ent = torch.empty(n, dtype=torch.float64, device=dev)
-                nb = _lib.lib().dqz_simple_update_workspace_bytes(n, rows, cols)
-                scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device=dev)
-                _lib.call("dqz_simple_update_ws", L.gptr, self._G.data_ptr(), self._lam.data_ptr(), edges.data_ptr(),
-                          first.data_ptr(), halves.data_ptr(), ranks.data_ptr(), n, EPS, self.max_chi, rows, cols,
-                          err.data_ptr(), ent.data_ptr(), scratch.data_ptr(), nb, stream)
-                self._err_chunks.append(err)
-                self._ent_chunks.append(ent)
-                self._seq_chunks.append(torch.tensor([op[9] for op in q2], dtype=torch.int64, device=dev))
+                runs.append((len(q2), put(np.array([op[3] for op in q2], dtype=np.int32)),
+                             put(np.array([op[4] for op in q2], dtype=np.uint8)), put(np.stack([op[5] for op in q2])),
+                             put(np.array([op[6] for op in q2], dtype=np.int32)),
+                             put(np.array([op[9] for op in q2], dtype=np.int64)), max(op[7] for op in q2),
+                             max(op[8] for op in q2)))
+        host = np.zeros(used, dtype=np.uint8)
+        for at, a in pieces:
+            host[at : at + a.nbytes] = np.ascontiguousarray(a).reshape(-1).view(np.uint8)
+        tables = torch.from_numpy(host).to(dev)
+        base = tables.data_ptr()
+        for run in runs:
+            if len(run) == 3:
+                n, nodes, gates = run
+                _lib.call("dqz_apply1", L.gptr, self._G.data_ptr(), base + nodes, base + gates, n, stream)
+                continue
+            n, edges, first, halves, ranks, seq, rows, cols = run
+            err = torch.empty(n, dtype=torch.float64, device=dev)
+            ent = torch.empty(n, dtype=torch.float64, device=dev)
+            nb = _lib.lib().dqz_simple_update_workspace_bytes(n, rows, cols)
+            scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device=dev)
+            _lib.call("dqz_simple_update_ws", L.gptr, self._G.data_ptr(), self._lam.data_ptr(), base + edges,
+                      base + first, base + halves, base + ranks, n, EPS, self.max_chi, rows, cols,
+                      err.data_ptr(), ent.data_ptr(), scratch.data_ptr(), nb, stream)
+            self._err_chunks.append(err)
+            self._ent_chunks.append(ent)
+            self._seq_chunks.append(tables[seq : seq + 8 * n].view(torch.int64).clone())
         self._rho_cache = None
 
     # ---------------------------------------------------------- regauge
@@ -332,26 +361,16 @@ class BPQuantumEmulator:
     def _random_messages(self):
         L = self._layout
         init = get_message_random_nonnegative_initializer(int(self._rng.integers(0, 2**31 - 1)))
+        # one matrix per bond dimension (the initializer re-seeds on every call), packed on the host
         mats = {}
-        by_half = []
-        for h in range(L.n_halves):
-            c = int(L.edge_chi[L.half_edge[h]])
+        arena = np.zeros(max(L.msg_elems, 1), dtype=np.complex128)
+        for h, c in enumerate(L.half_chi().tolist()):
             if c not in mats:
-                nd = L.nodes[L.half_node[h]]
-                e = L.edges[L.half_edge[h]]
-                mats[c] = torch.from_numpy(init((nd, e)))
-            by_half.append(mats[c])
-        n2e = L.pack_messages([m.to(L.device) for m in by_half]) if L.exact() else self._pack_msgs(by_half)
-        e2n = n2e.clone()
-        return n2e, e2n
-
-    def _pack_msgs(self, by_half):
-        L = self._layout
-        arena = torch.zeros(max(L.msg_elems, 1), dtype=torch.complex128)
-        for h, m in enumerate(by_half):
+                mats[c] = init((L.nodes[L.half_node[h]], L.edges[L.half_edge[h]])).reshape(-1)
             o = int(L.half_msg_off[h])
-            arena[o : o + m.numel()] = m.reshape(-1)
-        return arena.to(L.device)
+            arena[o : o + c * c] = mats[c]
+        n2e = torch.from_numpy(arena).to(L.device)
+        return n2e, n2e.clone()
 
     def _bp_loop(self, T, n2e, e2n, vd, G, lam):
         L = self._layout

@@ -91,7 +91,7 @@ class GraphLayout:
     # ------------------------------------------------------------- shapes
     def node_dims(self, v: int) -> List[int]:
         h0, k = self.node_half[v], self.degree[v]
-        return [int(self.edge_chi[self.half_edge[h0 + j]]) for j in range(k)]
+        return self.edge_chi[self.half_edge[h0 : h0 + k]].tolist()
 
     def node_shape(self, v: int):
         return tuple(self.node_dims(v)) + (int(self.phys[v]),)

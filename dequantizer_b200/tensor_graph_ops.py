@@ -13,6 +13,7 @@ Like the reference these methods replace entries of the dict they are given
 the previous ones are never written to.
 """
 
+import math
 from typing import Dict, Optional, Tuple
 
 import numpy as np
@@ -145,8 +146,8 @@ def simple_update_shapes(dims1, d1, i1, dims2, d2, i2, r, max_rank):
     """Host-side shape rule of tensor_ops.py:318-389: returns
     (rows1, rows2, cols, new bond dimension, full rank kk)."""
     chi = dims1[i1]
-    m1 = d1 * int(np.prod([c for j, c in enumerate(dims1) if j != i1]))
-    m2 = d2 * int(np.prod([c for j, c in enumerate(dims2) if j != i2]))
+    m1 = d1 * math.prod(c for j, c in enumerate(dims1) if j != i1)
+    m2 = d2 * math.prod(c for j, c in enumerate(dims2) if j != i2)
     k = chi * r
     kk = min(min(m1, k), min(m2, k))
     new = kk if max_rank is None else min(int(max_rank), kk)

@@ -71,9 +71,13 @@ def ising_sqrt_partition(
         init = get_potts_initializer(two, one)
         eng.load_tensors([init(n) for n in eng.topo.nodes])
         msg_init = get_message_random_nonnegative_initializer(key)
-        n2e = [msg_init((nd, e)) for nd, e in eng.topo.half_ids()]
-        e2n = [msg_init((e, nd)) for nd, e in eng.topo.half_ids()]
-        eng.load_messages(n2e, e2n)
+        # the initializer re-seeds on every call: one matrix per bond dimension, both directions alike
+        by_dim, n2e = {}, []
+        for nd, e in eng.topo.half_ids():
+            if e.dimension not in by_dim:
+                by_dim[e.dimension] = msg_init((nd, e))
+            n2e.append(by_dim[e.dimension])
+        eng.load_messages(n2e)
         hist, G, lam = eng.canonicalise(accuracy, max_iterations, graphed=graphed)
         rho = eng.densities()
         mag = float((2 * rho[:, 0, 0].real - 1).mean())
@@ -121,6 +125,7 @@ def run_eagle_simulation(
     em = BPQuantumEmulator(lattice, key, max_chi, per_regauging, accuracy, max_belief_propagation_iterations,
                            synchronous_update, traversal_type)
     rzz, rx = kicked_ising_gates(theta)
+    rzz = em.split_q2(rzz)
 
     def readout():
         if all_qubits:
