@@ -201,8 +201,7 @@ class BPEngine:
             m_off = [int(L.half_msg_off[h]) for h in h_off[:-1]] + [L.msg_elems]
             plan = []
             for lo, hi in zip(bounds[:-1], bounds[1:]):
-                ids = (torch.arange(h_off[lo], h_off[hi], dtype=torch.int32, device=L.device)
-                       if self.precision == "fp32" else torch.arange(lo, hi, dtype=torch.int32, device=L.device))
+                ids = torch.arange(lo, hi, dtype=torch.int32, device=L.device)
                 plan.append((lo, hi, t_off[lo], t_off[hi], m_off[lo], m_off[hi], ids))
             self._chunk_lists[chunks] = plan
         src_sel, edge_new, _ = topo.device_tables(L.device)
@@ -248,9 +247,9 @@ class BPEngine:
                           self.e2n.data_ptr(), n2e_new.data_ptr(), src_sel.data_ptr(), ids.data_ptr(), ids.numel(),
                           flag.data_ptr(), stream)
             elif self.precision == "fp32":
-                _lib.call("dqz_bp_node_update_k3", L.gptr, chi, 32, self.T.data_ptr(), self.n2e.data_ptr(),
-                          self.e2n.data_ptr(), n2e_new.data_ptr(), src_sel.data_ptr(), ids.data_ptr(), ids.numel(),
-                          flag.data_ptr(), stream)
+                _lib.call("dqz_bp_sweep_k3_c64", L.gptr, chi, self.T.data_ptr(), self.n2e.data_ptr(),
+                          self.e2n.data_ptr(), n2e_new.data_ptr(), e2n_new.data_ptr(), src_sel.data_ptr(),
+                          edge_new.data_ptr(), ids.data_ptr(), ids.numel(), flag.data_ptr(), stream)
             else:
                 _lib.call("dqz_bp_sweep_k3", L.gptr, chi, 1, self.T.data_ptr(), self.n2e.data_ptr(),
                           self.e2n.data_ptr(), n2e_new.data_ptr(), e2n_new.data_ptr(), src_sel.data_ptr(),
@@ -258,7 +257,7 @@ class BPEngine:
             down.wait_event(cur.record_event())
             with torch.cuda.stream(down):
                 out_n2e[ma:mb].copy_(n2e_new[ma:mb], non_blocking=True)
-        if self.T.dtype == torch.complex64:
+        if self.T_bf16 is not None:
             _lib.call("dqz_bp_edge_pass_c64", L.gptr, self.n2e.data_ptr(), n2e_new.data_ptr(), edge_new.data_ptr(),
                       e2n_new.data_ptr(), stream)
         if self.T_bf16 is not None:

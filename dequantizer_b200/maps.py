@@ -294,10 +294,13 @@ def bp_sweep(layout: GraphLayout, topo: Topology, T, n2e_old, e2n_old, n2e_new, 
                           e2n_old.data_ptr(), n2e_new.data_ptr(), src_sel.data_ptr(), nodes.data_ptr(),
                           nodes.numel(), flag.data_ptr(), stream)
         else:
-            for halves in levels:
-                _lib.call("dqz_bp_node_update_k3", layout.gptr, chi3, 32, T.data_ptr(), n2e_old.data_ptr(),
-                          e2n_old.data_ptr(), n2e_new.data_ptr(), src_sel.data_ptr(), halves.data_ptr(),
-                          halves.numel(), flag.data_ptr(), stream)
+            for nodes in topo.device_node_levels(layout.device):  # node update and edge pass in one launch
+                _lib.call("dqz_bp_sweep_k3_c64", layout.gptr, chi3, T.data_ptr(), n2e_old.data_ptr(),
+                          e2n_old.data_ptr(), n2e_new.data_ptr(), e2n_new.data_ptr(), src_sel.data_ptr(),
+                          edge_new.data_ptr(), nodes.data_ptr(), nodes.numel(), flag.data_ptr(), stream)
+            if mid_event is not None:
+                mid_event.record(torch.cuda.current_stream())
+            return
         if mid_event is not None:
             mid_event.record(torch.cuda.current_stream())
         _lib.call("dqz_bp_edge_pass_c64", layout.gptr, n2e_old.data_ptr(), n2e_new.data_ptr(), edge_new.data_ptr(),

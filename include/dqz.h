@@ -133,6 +133,13 @@ int dqz_bp_sweep_k3(const dqz_graph_t *g, int32_t max_chi, int32_t uniform, cons
                     const void *n2e_old, const void *e2n_old, void *n2e_new, void *e2n_new,
                     const uint8_t *src_sel, const uint8_t *edge_new, const int32_t *nodes, int32_t n_nodes,
                     int32_t raw, double *max_change, int32_t *error_flag, cudaStream_t stream);
+/* The same in FP32 (complex64 arenas; bonds all chi = 8 or 16, physical dimension
+ * 2): node update of the listed nodes and, with e2n_new, the edge pass. */
+int dqz_bp_sweep_k3_c64(const dqz_graph_t *g, int32_t chi, const void *tensors, const void *n2e_old,
+                        const void *e2n_old, void *n2e_new, void *e2n_new, const uint8_t *src_sel,
+                        const uint8_t *edge_new, const int32_t *nodes, int32_t n_nodes, int32_t *error_flag,
+                        cudaStream_t stream);
+
 
 /* Mixed-precision node update on tensor cores for the same shapes with
  * chi = 16: BF16 products, FP32 accumulation, complex64 messages. One CTA per
