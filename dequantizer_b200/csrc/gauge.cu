@@ -616,10 +616,12 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_distance_kernel(dqz_graph
     __syncthreads();
     // the trace norm from the eigenvalues (tridiagonal reduction, then counts or,
     // above bond 32, implicit QL; the staging area is free again for its vectors).
-    // Measured at 288 half-edges of bond 32:
-    // 672 us with QL, 504 us with counts (the sum over the slices is the rest).
-    const double t = ce <= 32 ? cta_trace_norm32(Rm, ce, ce, *reinterpret_cast<TraceNorm32Smem *>(U)) : herm_trace_norm(Rm, ce, ce, U, U + DQZ_MAX_CHI, reinterpret_cast<double *>(U + 2 * DQZ_MAX_CHI),
-                                     reinterpret_cast<double *>(U + 3 * DQZ_MAX_CHI), red);
+    // Measured at 288 half-edges of bond 32: 672 us with QL, 504 us with counts (R on
+    // the FP64 tensor cores, one CTA per SM for its registers: 523 us).
+    const double t = ce <= 32 ? cta_trace_norm32(Rm, ce, ce, *reinterpret_cast<TraceNorm32Smem *>(U))
+                              : herm_trace_norm(Rm, ce, ce, U, U + DQZ_MAX_CHI,
+                                                reinterpret_cast<double *>(U + 2 * DQZ_MAX_CHI),
+                                                reinterpret_cast<double *>(U + 3 * DQZ_MAX_CHI), red);
     if (tid == 0) partial[h] = t;
     __syncthreads();
   }
@@ -762,30 +764,56 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_distance_warp_kernel(
 }
 
 // ---------------------------------------------------------- symmetric gauge
-__global__ void __launch_bounds__(GAUGE_THREADS) symmetric_kernel(dqz_graph_t g, const cd *__restrict__ Tin,
-                                                                   const double *__restrict__ lambdas, double eps,
-                                                                   cd *Tout) {
+// Memory-bound: the square roots of the lambdas are taken once per node, not per
+// entry, and positions are 32-bit. Measured over the 21 calls of a kicked-Ising run
+// on the 127-qubit heavy-hex lattice (bonds growing to 32): 2.10 ms before, 0.57 ms
+// (0.64 ms with 1,024 threads a node).
+constexpr int SYM_THREADS = 512;
+__global__ void __launch_bounds__(SYM_THREADS) symmetric_kernel(dqz_graph_t g, const cd *__restrict__ Tin,
+                                                                const double *__restrict__ lambdas, double eps,
+                                                                cd *Tout) {
   __shared__ double red[48];
+  __shared__ double root[DQZ_MAX_DEGREE][DQZ_MAX_CHI];
   for (int v = blockIdx.x; v < g.n_nodes; v += gridDim.x) {
     NodeShape s;
     load_shape(g, v, s);
-    const double *lam[DQZ_MAX_DEGREE];
-    for (int f = 0; f < s.k; ++f) lam[f] = lambdas + g.edge_lam_off[g.half_edge[s.half0 + f]];
+    for (int i = threadIdx.x; i < s.k * DQZ_MAX_CHI; i += blockDim.x) {
+      const int f = i / DQZ_MAX_CHI, c = i % DQZ_MAX_CHI;
+      if (c < s.dims[f]) root[f][c] = sqrt(safe_truncate(lambdas[g.edge_lam_off[g.half_edge[s.half0 + f]] + c], eps));
+    }
+    __syncthreads();
     const cd *T = Tin + g.node_off[v];
     cd *O = Tout + g.node_off[v];
-    double n2 = 0.0;
-    for (long long i = threadIdx.x; i < s.size; i += blockDim.x) {
+    auto weight = [&](long long i) {
       double wt = 1.0;
-      for (int f = 0; f < s.k; ++f) wt *= sqrt(safe_truncate(lam[f][(i / s.stride[f]) % s.dims[f]], eps));
+      if (s.size < (1ll << 31)) {
+        unsigned x = (unsigned)i / (unsigned)s.d;  // from the last bond; multiplied from the first, as ever
+        double b[DQZ_MAX_DEGREE];
+#pragma unroll
+        for (int f = DQZ_MAX_DEGREE - 1; f >= 0; --f) {
+          if (f >= s.k) continue;
+          const unsigned q = (unsigned)s.dims[f], y = x / q;
+          b[f] = root[f][x - y * q];
+          x = y;
+        }
+#pragma unroll
+        for (int f = 0; f < DQZ_MAX_DEGREE; ++f)
+          if (f < s.k) wt *= b[f];
+      } else {
+        for (int f = 0; f < s.k; ++f) wt *= root[f][(i / s.stride[f]) % s.dims[f]];
+      }
+      return wt;
+    };
+    double n2 = 0.0;
+#pragma unroll 4
+    for (long long i = threadIdx.x; i < s.size; i += blockDim.x) {
+      const double wt = weight(i);
       n2 += cabs2(T[i]) * wt * wt;
     }
     n2 = block_sum(n2, red);
     const double inv = 1.0 / sqrt(n2);
-    for (long long i = threadIdx.x; i < s.size; i += blockDim.x) {
-      double wt = 1.0;
-      for (int f = 0; f < s.k; ++f) wt *= sqrt(safe_truncate(lam[f][(i / s.stride[f]) % s.dims[f]], eps));
-      O[i] = cscale(T[i], wt * inv);
-    }
+#pragma unroll 4
+    for (long long i = threadIdx.x; i < s.size; i += blockDim.x) O[i] = cscale(T[i], weight(i) * inv);
     __syncthreads();
   }
 }
@@ -1124,7 +1152,7 @@ extern "C" int dqz_symmetric_gauge(const dqz_graph_t *g, const void *tensors_in,
                                    void *tensors_out, cudaStream_t stream) {
   if (!g || !tensors_in || !lambdas || !tensors_out) return DQZ_ERR_ARG;
   if (g->n_nodes == 0) return DQZ_OK;
-  symmetric_kernel<<<g->n_nodes, GAUGE_THREADS, 0, stream>>>(*g, (const cd *)tensors_in, lambdas, eps,
+  symmetric_kernel<<<g->n_nodes, SYM_THREADS, 0, stream>>>(*g, (const cd *)tensors_in, lambdas, eps,
                                                               (cd *)tensors_out);
   DQZ_CHECK_LAUNCH();
   return DQZ_OK;

@@ -137,3 +137,24 @@ def test_distance_of_diagonal_zero_and_non_finite_tensors():
             assert not np.isfinite(part[h0:h0 + 3]).any()
         else:
             assert np.abs(part[h0:h0 + 3] - ref).max() < 1e-13
+
+
+@pytest.mark.parametrize("dims,phys", [((32,), 2), ((1, 31, 8), 3), ((2, 5), 1)])
+def test_symmetric_gauge(dims, phys):
+    """T times the square roots of the kept lambdas over its norm: a product of
+    three roots and one division, the norm's sum 65,536 / 512 terms a lane in
+    chains: 128 eps = 3e-14 of an entry, 1e-13."""
+    from dequantizer_b200 import _lib
+    L = layout_of(rr3(8, dims, phys))
+    rng = np.random.default_rng(4)
+    T = torch.from_numpy(rng.standard_normal(L.tensor_elems) + 1j * rng.standard_normal(L.tensor_elems)).cuda()
+    lam = torch.from_numpy(10.0 ** -rng.uniform(0, 12, L.lam_elems)).cuda()
+    out = torch.zeros_like(T)
+    _lib.call("dqz_symmetric_gauge", L.gptr, T.data_ptr(), lam.data_ptr(), 1e-10, out.data_ptr(), _lib.stream_handle())
+    for v, (t, o) in enumerate(zip(L.unpack_tensors(T), L.unpack_tensors(out))):
+        h0 = int(L.node_half[v])
+        for f in range(3):
+            le = L.lambda_view(lam, int(L.half_edge[h0 + f]))
+            t = t * torch.where(le > 1e-10, le, 0.0).sqrt().reshape([-1 if i == f else 1 for i in range(4)])
+        t = t / t.norm()
+        assert float(((o - t).abs() - 1e-13 * t.abs()).max()) <= 0.0
