@@ -430,7 +430,8 @@ __device__ __forceinline__ void warp_plan_item(const long long *pw, const cd *__
 // exact while x y < 2^30.
 // Bound by the levels' chain, and within a level by the SM's shared-memory port (five
 // items' operand loads at once). 16 warps: with 32 the registers spill. Measured on the
-// 6 x 6 x 6 lattice, bond 2 (206 levels, 5 half-edges each): 661 us, 1,750 us by slices.
+// 6 x 6 x 6 lattice, bond 2 (206 levels, 5 half-edges each): 572 us, 661 us with an
+// output at a time in the products, 1,750 us by slices.
 struct PlanWarp {
   long long pw[DQZ_PLAN_WORDS + 1];
   int4 bond[DQZ_MAX_DEGREE];    // stride R, dimension q, small_div's factors of R and q
@@ -483,7 +484,39 @@ __device__ __forceinline__ void plan_load_tensor(const PlanWarp &W, const cd *__
   cp_async_commit();
 }
 
-// Y = X x_f m over the whole tensor.
+// Y = X x_f m over the whole tensor, Q the bond's dimension: a lane takes whole
+// fibers (all Q entries along the bond, U fibers at a time), so each entry of X is
+// read once, and a row of m once for all of them. For bonds up to 4; above, Q U
+// entries a lane spill the registers.
+template <int Q, int U>
+__device__ __forceinline__ void plan_fibers(const int4 &bond, unsigned size, const cd *X, cd *Y, const cd *m) {
+  const unsigned R = (unsigned)bond.x, fR = (unsigned)bond.z, fibers = size / Q;
+  for (unsigned o0 = threadIdx.x & 31; o0 < fibers; o0 += 32 * U) {
+    cd x[U][Q];
+    unsigned at[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned o = o0 + 32 * u < fibers ? o0 + 32 * u : o0;
+      at[u] = o + small_div(o, fR) * (Q - 1) * R;
+#pragma unroll
+      for (int b = 0; b < Q; ++b) x[u][b] = X[at[u] + b * R];
+    }
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      cd row[Q];
+#pragma unroll
+      for (int b = 0; b < Q; ++b) row[b] = m[i * Q + b];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        cd acc = czero();
+#pragma unroll
+        for (int b = 0; b < Q; ++b) cfma(acc, row[b], x[u][b]);
+        if (o0 + 32 * u < fibers) Y[at[u] + i * R] = acc;
+      }
+    }
+  }
+}
+// The same for any bond, an output a time.
 template <int U>
 __device__ __forceinline__ void plan_product(const int4 &bond, unsigned size, const cd *X, cd *Y, const cd *m) {
   const unsigned R = (unsigned)bond.x, q = (unsigned)bond.y, fR = (unsigned)bond.z, fq = (unsigned)bond.w;
@@ -626,7 +659,13 @@ __global__ void __launch_bounds__(PLAN_THREADS) bp_sweep_whole_kernel(
       for (int f = e == 0 ? 1 : 0; f < k;) {
         const int after = f + 1 == e ? f + 2 : f + 1;
         const int4 nb = W.bond[after < k ? after : e];  // on its way during the product; the pairs' at the end
-        plan_product<4>(bond, size, cur, nxt, Ms + W.moff[f]);
+        const cd *m = Ms + W.moff[f];
+      switch (bond.y) {
+        case 2: plan_fibers<2, 2>(bond, size, cur, nxt, m); break;
+        case 3: plan_fibers<3, 2>(bond, size, cur, nxt, m); break;
+        case 4: plan_fibers<4, 1>(bond, size, cur, nxt, m); break;
+        default: plan_product<4>(bond, size, cur, nxt, m);
+      }
         bond = nb;
         f = after;
         __syncwarp();

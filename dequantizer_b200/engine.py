@@ -291,6 +291,8 @@ class BPEngine:
                 return len(self.topo.levels)  # the edge pass runs in the node update's launch (dqz_bp_sweep_k3)
             if len(self.topo.levels) > 1:
                 return 1  # every level and the edge pass in one cooperative launch (dqz_bp_sweep_levels)
+        if self.precision == "fp32":
+            return len(self.topo.levels)  # likewise (dqz_bp_sweep_k3_c64)
         return len(self.topo.levels) + 1
 
     def check(self) -> None:
