@@ -420,15 +420,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, MIN_BLOCKS)
     su_load_side(g, lambdas, hu, U);
     su_load_side(g, lambdas, hv, V);
     const int r = ranks[j];
-    // decided on the job's shapes before any update; the mark tells the
-    // global-scratch kernel (launched next) which jobs are done, since this
-    // launch changes the bond dimensions the decision reads
+    // decided on the job's shapes before any update (this launch changes the bond
+    // dimensions the decision reads), alike in both CTAs
     // chained: a launch before this one marked the jobs it did (their shapes
-    // have changed since); the others are decided here and marked when done
+    // have changed since); the others are decided here. Every thread of both
+    // CTAs reads the mark here, so it is written only at the end of the job,
+    // behind the cluster barriers that all of them pass: a mark written here
+    // could send a later warp, or the partner CTA, past a job the others are in.
     if (chained && done[j]) continue;
     const bool fits = suf_fits(U, V, r, max_rank, cap);
-    if (side == 0 && threadIdx.x == 0 && (fits || !chained)) done[j] = fits ? 1 : 0;
-    if (!fits) continue;  // left to the global-scratch kernel; same decision in both CTAs
+    if (!fits) {  // left to the global-scratch kernel, which reads the mark after this launch
+      if (!chained && side == 0 && threadIdx.x == 0) done[j] = 0;
+      continue;
+    }
     const SUSide &X = side ? V : U;
     SufDims D, Du, Dv;
     suf_dims(U, r, Du);
@@ -688,7 +692,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, MIN_BLOCKS)
     if (side == 0) {
       double *lam_out = lambdas + g.edge_lam_off[e];
       for (int c = tid; c < rank; c += nt) lam_out[c] = lam_sh[c];
-      if (tid == 0) g.edge_chi[e] = rank;
+      if (tid == 0) {
+        g.edge_chi[e] = rank;
+        done[j] = 1;
+      }
     }
     // the next job reads lambdas (this edge's, written by CTA 0) and edge_chi
     cluster.sync();
