@@ -5,12 +5,15 @@
 // sqrt(m_f)^-1 U, sqrt(m_b)^-1 conj(V). For positive definite messages any factor
 // m = L L^H serves, since sqrt(m) = L W with W unitary: with Cholesky factors,
 //   C' = L_f^H conj(L_b) = U' S V'^H   (the same S),
-//   G_f = sqrt(m_f)^-1 U = L_f^-H U',  G_b = sqrt(m_b)^-1 conj(V) = conj(L_f U') S^-1,
-// so two Hermitian eigendecompositions and the right singular vectors drop out,
-// leaving two 16-step factorisations, one triangular solve, and a one-sided
-// Jacobi iteration on the columns of C' alone. G_f S G_b^T = 1 holds to rounding
-// by construction; the columns of U' are orthogonal to the Jacobi tolerance
-// relative to their own norms, also for small singular values.
+//   G_f = sqrt(m_f)^-1 U = L_f^-H U',  G_b = sqrt(m_b)^-1 conj(V) = L_b^-H conj(V'),
+// so two Hermitian eigendecompositions drop out, leaving two 16-step
+// factorisations, two triangular solves and a one-sided Jacobi iteration on the
+// columns of C'. Both U' (columns orthogonal to the Jacobi tolerance relative to
+// their own norms) and V' (a product of rotations) are unitary to rounding,
+// also for small singular values. conj(L_f U') S^-1 equals G_b too, without V',
+// but its columns carry the rounding of C' over their own singular value, eps
+// s_max / s_j: with it the Vidal distance of the gauge (4-regular graph of 26
+// nodes, bond 2, lambdas down to 1.4e-6) was off by 3e-12 relative.
 //
 // The reference drops message eigenvalues up to eps. The factored form is exact
 // only when none are: |G_f|_F^2 = sum 1 / (eigenvalues of m_f) (and the same for
@@ -37,8 +40,8 @@ constexpr unsigned long long ES_MARK = 0x7ff80000000000e5ull;  // in lambda[0]: 
 
 struct EdgeSmem {
   cd L[2][ES_MAX * ES_LD];  // Cholesky factors, row-major, zero above the diagonal and from bond c on
-  cd X[ES_MAX * ES_LD];     // C', then the unit left singular vectors, column-major
-  double dinv[ES_MAX], s[ES_MAX];
+  cd X[ES_MAX * ES_LD];     // C', the unit left singular vectors, then the right ones, column-major
+  double dinv[2][ES_MAX], s[ES_MAX];
   int perm[ES_MAX];
 };
 
@@ -77,7 +80,7 @@ __device__ __forceinline__ bool edge_cholesky(EdgeSmem &S, const cd *mf, const c
       ok = ok && piv > eps;
       const double inv = fast_rsqrt(piv);  // piv > eps, or the edge is given up
       const cd l = r > j ? cscale(A[j], inv) : (r == j ? mk(piv * inv, 0.0) : czero());
-      if (r == j && side == 0) S.dinv[j] = inv;
+      if (r == j) S.dinv[side][j] = inv;
       L[r * ES_LD + j] = r < c ? l : czero();
       __syncwarp();
 #pragma unroll
@@ -93,21 +96,66 @@ __device__ __forceinline__ bool edge_cholesky(EdgeSmem &S, const cd *mf, const c
   return __all_sync(0xffffffffu, ok);
 }
 
+// One rotation of the columns x, y by this lane's rows.
+__device__ __forceinline__ void rotate_pair(cd (&x)[4], cd (&y)[4], const PhaseRot &R) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const cd p = cmul(x[i], R.ph), q = y[i];
+    x[i] = mk(R.cs * p.x - R.sn * q.x, R.cs * p.y - R.sn * q.y);
+    y[i] = mk(R.sn * p.x + R.cs * q.x, R.sn * p.y + R.cs * q.y);
+  }
+}
+
+// This lane's two seats in the Jacobi rounds: columns of the matrix, rows sub + 4 i.
+struct EdgeSeat {
+  int grp, sub, ct, cb;
+  bool seat, last, has_x, has_y;
+  __device__ __forceinline__ EdgeSeat(int c) {
+    const int lane = threadIdx.x & 31, np = c + (c & 1), npairs = np / 2;
+    grp = lane >> 2;
+    sub = lane & 3;
+    seat = grp < npairs;
+    last = grp == npairs - 1;
+    ct = grp == 0 ? 0 : grp + 1;  // rr_pair's step 0
+    cb = grp == 0 ? 1 : np - grp;
+    has_x = seat && ct < c;
+    has_y = seat && cb < c;
+  }
+  __device__ __forceinline__ void store(cd *X, const cd (&x)[4], const cd (&y)[4], double fx, double fy) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (has_x) X[ct * ES_LD + sub + 4 * i] = cscale(x[i], fx);
+      if (has_y) X[cb * ES_LD + sub + 4 * i] = cscale(y[i], fy);
+    }
+  }
+  // upper columns one seat down (seat 1's to seat 0's lower place), lower ones one up
+  __device__ __forceinline__ void move(cd (&x)[4], cd (&y)[4]) const {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const cd nx = shfl_cd(x[i], (lane + 4) & 31), ny = shfl_cd(y[i], (lane - 4) & 31), ky = y[i];
+      y[i] = grp == 0 ? nx : ny;
+      if (grp > 0) x[i] = last ? ky : nx;
+    }
+  }
+};
+
 // One-sided Jacobi on the columns of S.X (c x c): on return S.X holds the unit
-// left singular vectors, S.s the singular values. False when one is numerically
-// null (hestenes' rule).
-__device__ __forceinline__ bool edge_jacobi(EdgeSmem &S, int c) {
-  const int lane = threadIdx.x & 31, grp = lane >> 2, sub = lane & 3;
+// left singular vectors, S.s the singular values and vx, vy the right singular
+// vectors of this lane's seats. False when a value is numerically null
+// (hestenes' rule).
+__device__ __forceinline__ bool edge_jacobi(EdgeSmem &S, int c, const EdgeSeat &E, cd (&vx)[4], cd (&vy)[4]) {
+  const int sub = E.sub, ct = E.ct, cb = E.cb;
   const int np = c + (c & 1), npairs = np / 2;
   const double tol = 1.1e-16 * sqrt((double)c) * 2.0;
-  const bool seat = grp < npairs, last = grp == npairs - 1;
-  const int ct = grp == 0 ? 0 : grp + 1, cb = grp == 0 ? 1 : np - grp;  // rr_pair's step 0
-  const bool has_x = seat && ct < c, has_y = seat && cb < c;
+  const bool seat = E.seat, has_x = E.has_x, has_y = E.has_y;
   cd x[4], y[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     x[i] = has_x ? S.X[ct * ES_LD + sub + 4 * i] : czero();
     y[i] = has_y ? S.X[cb * ES_LD + sub + 4 * i] : czero();
+    vx[i] = mk(sub + 4 * i == ct ? 1.0 : 0.0, 0.0);
+    vy[i] = mk(sub + 4 * i == cb ? 1.0 : 0.0, 0.0);
   }
   double al, be;
   cd ga;
@@ -124,20 +172,12 @@ __device__ __forceinline__ bool edge_jacobi(EdgeSmem &S, int c) {
       PhaseRot R;
       if (rot && phase_rot(al, be, ga, R)) {
         rotated = true;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const cd p = cmul(x[i], R.ph), q = y[i];
-          x[i] = mk(R.cs * p.x - R.sn * q.x, R.cs * p.y - R.sn * q.y);
-          y[i] = mk(R.sn * p.x + R.cs * q.x, R.sn * p.y + R.cs * q.y);
-        }
+        rotate_pair(x, y, R);
+        rotate_pair(vx, vy, R);
       }
-      if (npairs > 1) {  // upper columns one seat down (seat 1's to seat 0's lower place), lower ones one up
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const cd nx = shfl_cd(x[i], (lane + 4) & 31), ny = shfl_cd(y[i], (lane - 4) & 31), ky = y[i];
-          y[i] = grp == 0 ? nx : ny;
-          if (grp > 0) x[i] = last ? ky : nx;
-        }
+      if (npairs > 1) {
+        E.move(x, y);
+        E.move(vx, vy);
       }
     }
     if (!__any_sync(0xffffffffu, rotated)) break;
@@ -147,17 +187,51 @@ __device__ __forceinline__ bool edge_jacobi(EdgeSmem &S, int c) {
   be = quad_sum(be);
   const double sa = sqrt(al), sb = sqrt(be), ia = 1.0 / sa, ib = 1.0 / sb;
   __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (has_x) S.X[ct * ES_LD + sub + 4 * i] = cscale(x[i], ia);
-    if (has_y) S.X[cb * ES_LD + sub + 4 * i] = cscale(y[i], ib);
-  }
+  E.store(S.X, x, y, ia, ib);
   if (sub == 0) {
     if (has_x) S.s[ct] = sa;
     if (has_y) S.s[cb] = sb;
   }
   __syncwarp();
   return __all_sync(0xffffffffu, (!has_x || al > null_thr) && (!has_y || be > null_thr));
+}
+
+// G = L^-H B diag(scale where mask, else 0) with B = S.X's columns in descending
+// order, conjugated for the b side; the squared norm of L^-H B over the warp. Lane
+// (half, j) holds the rows of parity `half` of column j.
+__device__ __forceinline__ double edge_solve(const EdgeSmem &S, int side, int c, unsigned mask, double scale, cd *G) {
+  const int lane = threadIdx.x & 31, j = lane & 15, half = lane >> 4;
+  const cd *L = S.L[side];
+  const double *dinv = S.dinv[side];
+  cd u[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    u[k] = j < c ? S.X[S.perm[j] * ES_LD + 2 * k + half] : czero();
+    if (side) u[k] = cconj(u[k]);
+  }
+#pragma unroll
+  for (int i = ES_MAX - 1; i >= 0; --i) {
+    if (i < c) {
+      const cd xi = cscale(shfl_cd(u[i >> 1], j + 16 * (i & 1)), dinv[i]);
+      if (half == (i & 1)) u[i >> 1] = xi;
+#pragma unroll
+      for (int k = 0; k < (i + 1) / 2; ++k) {
+        const int row = 2 * k + half;
+        const cd l = row < i ? L[i * ES_LD + row] : czero();
+        u[k] = csub(u[k], cmulc(l, xi));
+      }
+    }
+  }
+  double n = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int row = 2 * k + half;
+    if (j < c && row < c) {
+      n += cabs2(u[k]);
+      G[row * c + j] = (mask >> j) & 1u ? cscale(u[k], scale) : czero();
+    }
+  }
+  return warp_sum(n);
 }
 
 // One edge by the factored form; false (nothing written but possibly
@@ -172,54 +246,20 @@ __device__ __forceinline__ bool edge_svd_factored(EdgeSmem &S, const cd *mf, con
       t, [&](int i, int k) { return S.L[0][k * ES_LD + i]; }, [&](int k, int j) { return S.L[1][k * ES_LD + j]; });
   ctile_each(t, [&](int i, int j, cd v) { S.X[j * ES_LD + i] = v; });
   __syncwarp();
-  if (!edge_jacobi(S, c)) return false;
+  const EdgeSeat seats(c);
+  cd vx[4], vy[4];
+  if (!edge_jacobi(S, c, seats, vx, vy)) return false;
   warp_sort_desc(S.s, c, S.perm);
   const double sj = lane < c ? S.s[S.perm[lane]] : 0.0;
   const double l0 = sj / sqrt(warp_sum(sj * sj));
   const double kept = l0 > eps ? l0 : 0.0;
   const unsigned mask = __ballot_sync(0xffffffffu, lane < c && kept > eps);
   const double scale = 1.0 / sqrt((double)__popc(mask));
-  // G_b = conj(L_f U') / s, columns in descending order
-  t.clear();
-  cgemm<false, false, 2>(
-      t, [&](int i, int k) { return S.L[0][i * ES_LD + k]; },
-      [&](int k, int j) { return j < c ? S.X[S.perm[j] * ES_LD + k] : czero(); });
-  double nb = 0.0;
-  ctile_each(t, [&](int i, int j, cd v) {
-    if (i >= c || j >= c) return;
-    const cd x = cscale(cconj(v), 1.0 / S.s[S.perm[j]]);
-    nb += cabs2(x);
-    Gb[i * c + j] = (mask >> j) & 1u ? cscale(x, scale) : czero();
-  });
-  nb = warp_sum(nb);
-  // G_f = L_f^-H U': lane (half, j) holds the rows of parity `half` of column j
-  const int j = lane & 15, half = lane >> 4;
-  cd u[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) u[k] = j < c ? S.X[S.perm[j] * ES_LD + 2 * k + half] : czero();
-#pragma unroll
-  for (int i = ES_MAX - 1; i >= 0; --i) {
-    if (i < c) {
-      const cd xi = cscale(shfl_cd(u[i >> 1], j + 16 * (i & 1)), S.dinv[i]);
-      if (half == (i & 1)) u[i >> 1] = xi;
-#pragma unroll
-      for (int k = 0; k < (i + 1) / 2; ++k) {
-        const int row = 2 * k + half;
-        const cd l = row < i ? S.L[0][i * ES_LD + row] : czero();
-        u[k] = csub(u[k], cmulc(l, xi));
-      }
-    }
-  }
-  double nf = 0.0;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const int row = 2 * k + half;
-    if (j < c && row < c) {
-      nf += cabs2(u[k]);
-      Gf[row * c + j] = (mask >> j) & 1u ? cscale(u[k], scale) : czero();
-    }
-  }
-  nf = warp_sum(nf);
+  const double nf = edge_solve(S, 0, c, mask, scale, Gf);
+  __syncwarp();
+  seats.store(S.X, vx, vy, 1.0, 1.0);
+  __syncwarp();
+  const double nb = edge_solve(S, 1, c, mask, scale, Gb);
   const double limit = 0.5 / eps;
   if (!(nf < limit) || !(nb < limit)) return false;
   if (lane < c) lam[lane] = kept;
