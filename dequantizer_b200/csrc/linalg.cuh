@@ -45,29 +45,24 @@ __device__ __forceinline__ void rr_pair(int step, int i, int np, int &p, int &q)
 
 // The rotation that zeroes c in the Hermitian 2x2 [[a, c], [conj(c), b]] (a, b
 // real): J = D R, D = diag(ph, 1) with ph = c / |c|, R = [[cs, sn], [-sn, cs]],
-// t = sn / cs, ac = |c|. False when c is negligible.
-// The tangent is only a direction: a relative error of 1e-7 leaves 1e-7 of c,
-// which the next sweep removes, so it is formed in FP32; cs is then 1 / sqrt(1 +
-// t^2) of that very t, and ph the normalised c, both in FP64, so J is unitary
-// to rounding. This runs per pair and step as one dependent chain.
+// t = sn / cs = sign / (|zeta| + sqrt(1 + zeta^2)), zeta = (b - a) / 2 |c|. False
+// when c is negligible. This runs per pair and step as one dependent chain, hence
+// fast_rsqrt and fast_rcp (within 2 ulp; J is unitary to that) where their range
+// allows, CUDA's functions outside it.
 struct PhaseRot {
   cd ph;
-  double cs, sn, t, ac;
+  double cs, sn, t;
 };
 __device__ __forceinline__ bool phase_rot(double a, double b, cd c, PhaseRot &r) {
   const double ac2 = cabs2(c);
-  if (!(ac2 > 1e-290 && ac2 < 1e290)) return false;
-  const double inv = fast_rsqrt(ac2);
-  const double zeta = (b - a) * 0.5 * inv;
-  const float z = (float)fabs(zeta);
-  // t = 1 / (|zeta| + sqrt(1 + zeta^2)); |zeta| = |b - a| / 2 |c| is below 1e33 for a pair
-  // above the convergence thresholds
-  const float tf = z > 1e8f ? __fdividef(0.5f, z * 1e-8f) * 1e-8f : __fdividef(1.0f, z + __fsqrt_rn(fmaf(z, z, 1.0f)));
-  r.t = zeta >= 0.0 ? (double)tf : -(double)tf;
+  if (!(ac2 > 1e-300)) return false;
+  const double inv = fast_range(ac2) ? fast_rsqrt(ac2) : rsqrt(ac2);
+  const double zeta = (b - a) * 0.5 * inv, z = fabs(zeta), q = fma(z, z, 1.0);
+  const double t = q <= 1e290 ? fast_rcp(fma(q, fast_rsqrt(q), z)) : 0.5 / z;  // sqrt(1 + zeta^2) = |zeta| there
+  r.t = copysign(t, zeta);
   r.cs = fast_rsqrt(fma(r.t, r.t, 1.0));
   r.sn = r.t * r.cs;
   r.ph = mk(c.x * inv, c.y * inv);
-  r.ac = ac2 * inv;
   return true;
 }
 
