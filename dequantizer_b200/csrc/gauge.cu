@@ -25,7 +25,8 @@ constexpr size_t SMEM_LIMIT = 200 * 1024;
 constexpr int WARP_MAX_CHI = 16;     // largest bond of the one-warp kernels
 constexpr int WARP_ROTS = 17;        // rotation slots per warp (n / 2 + 1 for n <= 32)
 constexpr size_t WARP_BLOCK_SMEM = 96 * 1024;
-constexpr int SCRATCH_GRID = 148 * 4;
+constexpr int SM_COUNT = 148;
+constexpr int SCRATCH_GRID = SM_COUNT * 4;
 
 // Left to another kernel (edges: in lambda[0]; nodes: in rho[0]).
 __device__ __forceinline__ bool is_marked(double x) { return __double_as_longlong(x) == (long long)ES_MARK; }
@@ -156,8 +157,8 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_edges_kernel(dqz_graph_t 
 
 // One warp per edge (chi <= WARP_MAX_CHI), the factored form (edge_svd.cuh);
 // edges it does not cover get ES_MARK in lambda[0]. Measured at 1,536 edges of
-// bond 16 (random 3-regular graph, 1,024 nodes): 116 us, 1,442 us with the
-// eigendecompositions.
+// bond 16 (random 3-regular graph, 1,024 nodes): 193 us, 1,572 us with the
+// eigendecompositions; at bond 3 41 and 68 us; at bond 2 21 and 20 us.
 constexpr int ES_WARPS = 4;
 __global__ void __launch_bounds__(32 * ES_WARPS, 4) vidal_edges_factored_kernel(dqz_graph_t g,
                                                                                  const cd *__restrict__ n2e,
@@ -180,7 +181,19 @@ __global__ void __launch_bounds__(32 * ES_WARPS, 4) vidal_edges_factored_kernel(
   }
 }
 
-// One CTA per edge (WARP_MAX_CHI < max_chi <= RJ_MAX); the few it leaves run the
+// One CTA per edge, by edge_svd_cta; where it does not apply, marked.
+__device__ __forceinline__ void cta_edge(const dqz_graph_t &g, EdgeCtaSmem &S, int e, const cd *n2e, double eps,
+                                         cd *orth, double *lambdas, int max_chi) {
+  const int c = g.edge_chi[e];
+  double *lam = lambdas + g.edge_lam_off[e];
+  const long long of = g.half_msg_off[g.edge_half[2 * e]], ob = g.half_msg_off[g.edge_half[2 * e + 1]];
+  const bool fits = c <= max_chi;
+  const bool done = fits && edge_svd_cta(S, n2e + of, n2e + ob, c, eps, orth + of, orth + ob, lam);
+  if (!done && threadIdx.x == 0)
+    lam[0] = __longlong_as_double((long long)(fits ? ES_MARK : 0x7ff8000000000000ull));
+}
+
+// Every edge (WARP_MAX_CHI < max_chi <= RJ_MAX); the few it leaves run the first
 // kernel above. Bound by the Jacobi rounds' latency (31 of about 1,200 cycles a
 // sweep, two iterations after another). Measured at 144 edges of bond 32: 768 us,
 // 3,433 us with two-sided rotations and C formed in the original basis.
@@ -189,15 +202,31 @@ __global__ void __launch_bounds__(EC_THREADS) vidal_edges_cta_kernel(dqz_graph_t
                                                                      const int32_t *__restrict__ sel, int total) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   EdgeCtaSmem &S = *reinterpret_cast<EdgeCtaSmem *>(smem_raw);
-  for (int it = blockIdx.x; it < total; it += gridDim.x) {
-    const int e = sel ? sel[it] : it;
-    const int c = g.edge_chi[e];
-    double *lam = lambdas + g.edge_lam_off[e];
-    const long long of = g.half_msg_off[g.edge_half[2 * e]], ob = g.half_msg_off[g.edge_half[2 * e + 1]];
-    const bool fits = c <= max_chi;
-    const bool done = fits && edge_svd_cta(S, n2e + of, n2e + ob, c, eps, orth + of, orth + ob, lam);
-    if (!done && threadIdx.x == 0)
-      lam[0] = __longlong_as_double((long long)(fits ? ES_MARK : 0x7ff8000000000000ull));
+  for (int it = blockIdx.x; it < total; it += gridDim.x)
+    cta_edge(g, S, sel ? sel[it] : it, n2e, eps, orth, lambdas, max_chi);
+}
+
+// The edges that the factored kernel marked (rank-deficient messages: the leaves
+// of a graph), each by a whole CTA. Block b looks after the edges b, b + grid, ..
+__global__ void __launch_bounds__(EC_THREADS) vidal_edges_marked_kernel(dqz_graph_t g, const cd *__restrict__ n2e,
+                                                                        double eps, cd *orth, double *lambdas,
+                                                                        int max_chi, const int32_t *__restrict__ sel,
+                                                                        int total) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  EdgeCtaSmem &S = *reinterpret_cast<EdgeCtaSmem *>(smem_raw);
+  __shared__ int list[EC_THREADS];
+  __shared__ int found;
+  for (int base = blockIdx.x; base < total; base += EC_THREADS * gridDim.x) {
+    __syncthreads();
+    if (threadIdx.x == 0) found = 0;
+    __syncthreads();
+    const int it = base + threadIdx.x * gridDim.x;
+    if (it < total) {
+      const int e = sel ? sel[it] : it;
+      if (is_marked(lambdas[g.edge_lam_off[e]])) list[atomicAdd(&found, 1)] = e;
+    }
+    __syncthreads();
+    for (int i = 0; i < found; ++i) cta_edge(g, S, list[i], n2e, eps, orth, lambdas, max_chi);
   }
 }
 
@@ -228,10 +257,10 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_edges_warp_kernel(dqz_gra
     const int h0 = g.edge_half[2 * e], h1 = g.edge_half[2 * e + 1];
     const int c = g.edge_chi[e];
     double *lam = lambdas + g.edge_lam_off[e];
-    // the factored kernel before this one did every edge it did not mark
-    const unsigned long long mark = (unsigned long long)__double_as_longlong(lam[0]);
+    // the kernels before this one did every edge that is not marked
+    const bool marked = is_marked(lam[0]);
     __syncwarp();
-    if (mark != ES_MARK) continue;
+    if (!marked) continue;
     const cd *mf = n2e + g.half_msg_off[h0];
     const cd *mb = n2e + g.half_msg_off[h1];
     for (int i = lane; i < c * c; i += 32) {
@@ -1042,6 +1071,20 @@ extern "C" int dqz_vidal_edges(const dqz_graph_t *g, const void *n2e, double eps
     vidal_edges_factored_kernel<<<(total + ES_WARPS - 1) / ES_WARPS, 32 * ES_WARPS, ES_WARPS * sizeof(EdgeSmem),
                                   stream>>>(*g, (const cd *)n2e, eps, (cd *)orth, lambdas, max_chi, edges, total);
     DQZ_CHECK_LAUNCH();
+    // Marked edges: a CTA ends one sooner, but 148 run at a time; a warp each, a few
+    // thousand run side by side. How many there are is not known here, so a CTA takes
+    // them where it is the faster for all edges marked. Measured, us, CTA / warp: 144
+    // edges with two marked, bond 2 37 / 31, 3 59 / 71, 8 129 / 218, 16 306 / 951; all
+    // marked, bond 3 39 / 60, 16 203 / 1,388; 1,536 edges all marked, bond 8 689 / 331,
+    // 12 1,291 / 1,401, 16 1,745 / 2,932; 12,285 edges all marked, bond 12 9,891 / 7,284,
+    // 16 13,201 / 18,743.
+    if (max_chi > 14 || (max_chi > 2 && total <= 2 * SM_COUNT)) {
+      DQZ_SMEM_ATTR_ONCE(vidal_edges_marked_kernel, SMEM_LIMIT);
+      const int most = 3 * SM_COUNT;  // resident at once
+      vidal_edges_marked_kernel<<<total < most ? total : most, EC_THREADS, sizeof(EdgeCtaSmem), stream>>>(
+          *g, (const cd *)n2e, eps, (cd *)orth, lambdas, max_chi, edges, total);
+      DQZ_CHECK_LAUNCH();
+    }
     DQZ_SMEM_ATTR_ONCE(vidal_edges_warp_kernel, SMEM_LIMIT);
     vidal_edges_warp_kernel<<<(total + wpb - 1) / wpb, 32 * wpb, wpb * per, stream>>>(
         *g, (const cd *)n2e, eps, (cd *)orth, lambdas, max_chi, edges, total);
