@@ -213,9 +213,12 @@ __device__ __forceinline__ void reg_apply_q(cd (&x)[CPW][ROWS], const cd *__rest
 // rotation -> columns that bounds a round. On entry X holds the matrix; on
 // return its columns are u_j (zero for a numerically null one, s_j = 0) and V
 // holds the right singular vectors.
-// A sweep whose rotated pairs all had |cos| below 1e-9 ends the iteration: what
-// its rotations leave is below 1e-16 (1e-7 of the scalar products by the FP32
-// tangent, 1e-18 by second-order terms), as a further sweep would only confirm.
+// A sweep whose rotated pairs all had |cos| below 1e-9 and turned by less than
+// 1e-8 ends the iteration: a rotation gives back at most sin |cos| of what others
+// removed, so 2 n of them leave less than 64e-17, below the tolerance, and a further
+// sweep would only confirm. The angle matters: columns of equal norm turn by up to
+// 45 degrees however small their |cos| (with the first rule alone the gauge of a
+// message 1 + 1e-11 H was off by 2e-11).
 // Measured on the simple update's 32 x 32 cores: columns in registers moved from
 // seat to seat by shuffles (64 of about 9 cycles a round) 2,300 cycles a round and
 // 380 us for a launch of one core; this form 210 us.
@@ -326,7 +329,7 @@ static __device__ void cta_jacobi(cd *X, cd *V, int ld, int n, double *s, Jacobi
         PhaseRot R;
         const bool rot = live && al > null_thr && be > null_thr && g2 > tol * tol * ab && phase_rot(al, be, ga, R);
         if (rot) {
-          more |= g2 > 1e-18 * ab;
+          more |= g2 > 1e-18 * ab || fabs(R.t) > 1e-8;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const cd t = cmul(x[i], R.ph);
