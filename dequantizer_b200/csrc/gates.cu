@@ -801,9 +801,12 @@ extern "C" int dqz_simple_update_ws(const dqz_graph_t *g, void *tensors, double 
     if (st != DQZ_OK) return st;
     chained = 1;
   }
-  const bool larger = !chained || max_rows / 2 > 256 || max_cols > 32;  // a job may be above the register form
+  // Jobs above the register form can't be told from max_rows and max_cols (it also limits
+  // the rows without the physical index, the bond times the physical dimension and the
+  // rows of S), so the cluster forms are launched wherever they may have a job; one
+  // that finds every mark set ends in a few microseconds.
   const int pairs = n < sms / 2 ? n : sms / 2;  // one CTA per SM, two per cluster
-  if (larger && max_rows >= SUF_MIN_ROWS && (knob == 4 || (knob == 0 && n > sms))) {
+  if (max_rows >= SUF_MIN_ROWS && (knob == 4 || (knob == 0 && n > sms))) {
     // large batches (and knob 4): every 256-row job on the global-workspace
     // cluster form, 256 threads a CTA, two clusters per SM pair (measured at
     // bond 16: 3,924 jobs in 35.4 ms against 40.2 ms on the one-CTA kernel;
@@ -815,7 +818,7 @@ extern "C" int dqz_simple_update_ws(const dqz_graph_t *g, void *tensors, double 
                                     eps, max_rank, err, entropy, su_cluster_cap(max_rows, max_cols), marks,
                                     job_scratch, chained);
     DQZ_CHECK_LAUNCH();
-  } else if (larger && max_rows >= SUF_MIN_ROWS && (n <= sms || knob == 2) && knob != 1) {
+  } else if (max_rows >= SUF_MIN_ROWS && (n <= sms || knob == 2) && knob != 1) {
     auto *onchip = simple_update_onchip_kernel<SUF_THREADS, 1>;
     DQZ_SMEM_ATTR_ONCE(onchip, SUF_SMEM_MAX);
     const long long cap = (long long)(SUF_SMEM_MAX / sizeof(cd));
