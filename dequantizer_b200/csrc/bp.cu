@@ -32,12 +32,16 @@ __device__ __forceinline__ const cd *incoming_msg(const dqz_graph_t &g, int hf, 
 // Column a of the unnormalised outgoing message of bond e of a node (tensor
 // Tv, shape s): out[ap][a] = sum_x conj(T_slice(ap)[x]) Y_a[x], with Y_a the
 // bond-e slice a contracted with the k-1 incoming messages; `put(ap, value)`
-// stores each entry. bufA / bufB hold two slices. Whole CTA; ends with a barrier.
-template <typename Put>
+// stores each entry. bufA / bufB hold two slices. The message at a half-edge h with
+// fresh(h) is divided by its trace in `staged`. Whole CTA; ends with a barrier.
+struct NeverFresh {
+  __device__ __forceinline__ bool operator()(int) const { return false; }
+};
+template <typename Put, typename Fresh = NeverFresh>
 __device__ __forceinline__ void node_slice_column(const dqz_graph_t &g, const cd *__restrict__ Tv, const NodeShape &s,
                                                   int e, const cd *n2e_old, const cd *e2n_old, const cd *n2e_new,
                                                   const uint8_t *__restrict__ src_sel, int a, cd *bufA, cd *bufB,
-                                                  Put put, cd *staged = nullptr) {
+                                                  Put put, cd *staged = nullptr, Fresh fresh = Fresh()) {
   const int ce = s.dims[e];
   const long long Re = s.stride[e];
   const long long P = s.size / ce;
@@ -64,7 +68,7 @@ __device__ __forceinline__ void node_slice_column(const dqz_graph_t &g, const cd
     const int q = s.dims[f];
     const long long R = P / Lj / q;
     const cd *m = incoming_msg(g, s.half0 + f, n2e_old, e2n_old, n2e_new, src_sel);
-    if (staged && src_sel[s.half0 + f] == DQZ_SRC_N2E_NEW) {  // not yet normalised: divide by the trace
+    if (fresh(s.half0 + f)) {
       cd tr = czero();
       for (int i = 0; i < q; ++i) tr = cadd(tr, __ldcg(m + i * q + i));
       for (int i = threadIdx.x; i < q * q; i += blockDim.x) staged[i] = cdiv(__ldcg(m + i), tr);
@@ -155,12 +159,6 @@ __global__ void __launch_bounds__(BP_THREADS) bp_node_generic(dqz_graph_t g, con
 // this entry bit for bit.
 constexpr int SL_MIN_CHI = 8;
 
-__device__ __forceinline__ const cd *sl_source(const dqz_graph_t &g, int hf, const cd *n2e_old, const cd *e2n_old,
-                                               const cd *n2e_new, const uint8_t *src_sel, bool &fresh) {
-  fresh = src_sel[hf] == DQZ_SRC_N2E_NEW;
-  return incoming_msg(g, hf, n2e_old, e2n_old, n2e_new, src_sel);
-}
-
 __global__ void __launch_bounds__(SL_THREADS, 2) bp_node_slices(dqz_graph_t g, const cd *__restrict__ T,
                                                              const cd *n2e_old, const cd *e2n_old, cd *n2e_new,
                                                              const uint8_t *__restrict__ src_sel,
@@ -183,9 +181,10 @@ __global__ void __launch_bounds__(SL_THREADS, 2) bp_node_slices(dqz_graph_t g, c
     it.T = Tv;
     it.Re = (unsigned)s.stride[e];
     sl_load(it, buf);
-    bool fx = false, fy = false;  // earlier levels' messages are normalised already
-    const cd *mx = it.g.nb > 0 ? sl_source(g, s.half0 + it.g.fx, n2e_old, e2n_old, n2e_new, src_sel, fx) : nullptr;
-    const cd *my = it.g.nb > 1 ? sl_source(g, s.half0 + it.g.fy, n2e_old, e2n_old, n2e_new, src_sel, fy) : nullptr;
+    const cd *mx =
+        it.g.nb > 0 ? incoming_msg(g, s.half0 + it.g.fx, n2e_old, e2n_old, n2e_new, src_sel) : nullptr;
+    const cd *my =
+        it.g.nb > 1 ? incoming_msg(g, s.half0 + it.g.fy, n2e_old, e2n_old, n2e_new, src_sel) : nullptr;
     sl_columns(it, mx, false, my, false, buf, buf + SL_BUF, [&](int ap, int a, cd val) { dst[ap * ce + a] = val; });
     return;
   }
@@ -808,8 +807,9 @@ struct SweepItem {
 // computes them (nodes outside that form: node_slice_column per slice). A grid
 // barrier closes a level. The messages stay unnormalised until the end: readers of
 // this sweep's messages divide by the trace as they stage them, so a level needs
-// no second barrier; then every message is divided in place, a barrier, and the
-// edge pass. Bit-identical to the per-level launches.
+// no second barrier; then every listed message is divided in place, a barrier, and
+// the edge pass. Messages of half-edges that no level lists are as the caller left
+// them, for readers too. Bit-identical to the per-level launches.
 // Bound by the levels' chain: an item at bond 32 reads 1 MB of T through L2 (16 k
 // cycles an SM) and a level has 16 to 194 of them.
 // Measured at bond 32 on the 127-qubit heavy-hex lattice (72 levels): 1,746 us;
@@ -830,6 +830,16 @@ __global__ void __launch_bounds__(SL_THREADS, 2) bp_sweep_sliced_kernel(
   // of T is on its way before the barrier that opens the level.
   __shared__ SweepItem table[SL_LEVELS];
   __shared__ SweepItem other;  // further items of a level, and levels beyond the table
+  const int n_listed = level_off[n_levels];
+  const bool all_listed = n_listed >= g.n_halves;
+  auto computed = [&](int hf) {  // the message read at hf is one that this launch computes
+    if (src_sel[hf] != DQZ_SRC_N2E_NEW) return false;
+    if (all_listed) return true;
+    const int tw = g.half_twin[hf];
+    for (int i = 0; i < n_listed; ++i)
+      if (halves[i] == tw) return true;
+    return false;
+  };
   auto look_up = [&](int item, SweepItem &d) {
     d.item = item;
     d.h = item_half[item];
@@ -845,9 +855,12 @@ __global__ void __launch_bounds__(SL_THREADS, 2) bp_sweep_sliced_kernel(
     d.dst = n2e_new + g.half_msg_off[d.h];
     d.Re = (unsigned)s.stride[e];
     d.fast = sl_geometry(s, e, d.g);
-    d.fx = d.fy = false;
-    d.mx = d.fast && d.g.nb > 0 ? sl_source(g, s.half0 + d.g.fx, n2e_old, e2n_old, n2e_new, src_sel, d.fx) : nullptr;
-    d.my = d.fast && d.g.nb > 1 ? sl_source(g, s.half0 + d.g.fy, n2e_old, e2n_old, n2e_new, src_sel, d.fy) : nullptr;
+    const bool x = d.fast && d.g.nb > 0, y = d.fast && d.g.nb > 1;
+    const int hx = x ? s.half0 + d.g.fx : d.h, hy = y ? s.half0 + d.g.fy : d.h;
+    d.fx = x && computed(hx);
+    d.fy = y && computed(hy);
+    d.mx = x ? incoming_msg(g, hx, n2e_old, e2n_old, n2e_new, src_sel) : nullptr;
+    d.my = y ? incoming_msg(g, hy, n2e_old, e2n_old, n2e_new, src_sel) : nullptr;
   };
   for (int lv = threadIdx.x; lv < n_levels && lv < SL_LEVELS; lv += blockDim.x) {
     table[lv].begin = item_off[lv] + (int)blockIdx.x;
@@ -893,13 +906,13 @@ __global__ void __launch_bounds__(SL_THREADS, 2) bp_sweep_sliced_kernel(
           sl_load(it, buf);
         }
       } else {
-        // every fresh message is divided by its trace in a staged copy behind the two slices
+        // every message of this launch is divided by its trace in a staged copy behind the two slices
         NodeShape s;
         load_shape(g, g.half_node[d.h], s);
         for (int b = 0; b < d.n; ++b)
           node_slice_column(g, d.T, s, d.h - s.half0, n2e_old, e2n_old, n2e_new, src_sel, d.a0 + b, buf,
                             buf + max_slice, [&](int ap, cd val) { dst[ap * ce + d.a0 + b] = val; },
-                            buf + 2 * max_slice);
+                            buf + 2 * max_slice, computed);
       }
     }
     if (lv + 1 < n_levels && lv + 1 < SL_LEVELS && table[lv + 1].begin < table[lv + 1].end) {
@@ -911,8 +924,8 @@ __global__ void __launch_bounds__(SL_THREADS, 2) bp_sweep_sliced_kernel(
       return;
     }
   }
-  for (int h = blockIdx.x; h < g.n_halves; h += gridDim.x) {
-    const int e = g.half_edge[h];
+  for (int i = blockIdx.x; i < n_listed; i += gridDim.x) {
+    const int h = halves[i], e = g.half_edge[h];
     if (e < 0) continue;
     cd *m = n2e_new + g.half_msg_off[h];
     normalise_by_trace(m, m, g.edge_chi[e], trace_sh);

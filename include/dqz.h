@@ -216,8 +216,9 @@ int dqz_bp_sweep_planned(const dqz_graph_t *g, const void *tensors, const void *
  * a block of slices of its bond, item_slice[i] = first slice + (number << 16)
  * (number 0: one), for i in item_off[l] .. item_off[l+1], covering every slice of
  * every half-edge of the level, spread over the grid. Each writes its columns
- * of the unnormalised message; readers divide by the trace, and all messages
- * are divided at the end, before the edge pass. Bit-identical to the per-level
+ * of the unnormalised message; readers divide by the trace, and the messages of
+ * `halves` are divided at the end, before the edge pass; those of half-edges that
+ * no level lists stay as they are in n2e_new. Bit-identical to the per-level
  * launches; max_items bounds the items of one level. */
 int dqz_bp_sweep_sliced(const dqz_graph_t *g, const void *tensors, const void *n2e_old, const void *e2n_old,
                         void *n2e_new, void *e2n_new, const uint8_t *src_sel, const uint8_t *edge_new,
