@@ -812,9 +812,12 @@ struct SweepItem {
 // them, for readers too. Bit-identical to the per-level launches.
 // Bound by the levels' chain: an item at bond 32 reads 1 MB of T through L2 (16 k
 // cycles an SM) and a level has 16 to 194 of them.
-// Measured at bond 32 on the 127-qubit heavy-hex lattice (72 levels): 1,746 us;
-// one slice an item and generic arithmetic 3,252 us, without the table 2,107 us.
-__global__ void __launch_bounds__(SL_THREADS, 2) bp_sweep_sliced_kernel(
+// One CTA per SM: 120 KB with the table, and 217 registers a thread (128, for a
+// second one that never fits, spilled).
+// Measured at bond 32 on the 127-qubit heavy-hex lattice (72 levels): 1,677 us, 1,838 us
+// with the spills; one slice an item and generic arithmetic 3,252 us, without the
+// table 2,107 us.
+__global__ void __launch_bounds__(SL_THREADS) bp_sweep_sliced_kernel(
     dqz_graph_t g, const cd *__restrict__ T, const cd *n2e_old, const cd *e2n_old, cd *n2e_new, cd *e2n_new,
     const uint8_t *__restrict__ src_sel, const uint8_t *__restrict__ edge_new, const int32_t *__restrict__ halves,
     const int32_t *__restrict__ level_off, const int32_t *__restrict__ item_half,

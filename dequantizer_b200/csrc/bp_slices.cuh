@@ -13,7 +13,8 @@
 //
 // Bound: per slice of 32 x 32 x 2 the two mode products take 2,048 m8n8k4 (8.2 k
 // cycles of an SM) and the contraction 262 k multiply-adds (4.1 k) against 1 MB of
-// T; blocks of two slices halve that traffic and let two CTAs share an SM.
+// T; blocks of two slices halve that traffic and let two CTAs of the node update
+// share an SM (106 KB each; the one-launch sweep's table of levels adds 14 KB).
 // Measured (127-qubit heavy-hex lattice, bond 32, all 144 half-edges in one launch):
 // 425 us against 3,128 us of the generic form. Lanes as a' with rows of T read
 // whole, for the bonds whose entries lie close together, took 557 us.
