@@ -20,6 +20,7 @@ using namespace dqz;
 namespace {
 
 constexpr int BP_THREADS = 256;
+static_assert(BP_THREADS == SL_THREADS, "the one-launch sweep runs both forms");
 
 __device__ __forceinline__ const cd *incoming_msg(const dqz_graph_t &g, int hf, const cd *n2e_old, const cd *e2n_old,
                                                   const cd *n2e_new, const uint8_t *src_sel) {
@@ -757,23 +758,61 @@ __device__ __forceinline__ bool grid_barrier(unsigned *sync, unsigned &gen, int 
   return ok_sh != 0;
 }
 
+// n2e_new[h] by the whole CTA as bp_node_slices and bp_trace_kernel compute it: its
+// blocks of slices one after another (nodes outside that form: node_update_half).
+// Ends with a barrier.
+__device__ __forceinline__ void node_update_half_slices(const dqz_graph_t &g, const cd *__restrict__ T,
+                                                        const cd *n2e_old, const cd *e2n_old, cd *n2e_new,
+                                                        const uint8_t *__restrict__ src_sel, int h, cd *smem,
+                                                        int max_slice, int max_chi, cd &trace_sh) {
+  const int v = g.half_node[h];
+  NodeShape s;
+  load_shape(g, v, s);
+  const int e = h - s.half0;
+  SliceItem it;
+  if (!sl_geometry(s, e, it.g)) {
+    cd *bufA = smem + (long long)max_chi * max_chi;
+    node_update_half(g, T, n2e_old, e2n_old, n2e_new, src_sel, h, smem, bufA, bufA + max_slice, trace_sh);
+    return;
+  }
+  const int most = sl_count(it.g), ce = it.g.ce;
+  cd *dst = n2e_new + g.half_msg_off[h];
+  it.T = T + g.node_off[v];
+  it.Re = (unsigned)s.stride[e];
+  const cd *mx = it.g.nb > 0 ? incoming_msg(g, s.half0 + it.g.fx, n2e_old, e2n_old, n2e_new, src_sel) : nullptr;
+  const cd *my = it.g.nb > 1 ? incoming_msg(g, s.half0 + it.g.fy, n2e_old, e2n_old, n2e_new, src_sel) : nullptr;
+  for (it.a0 = 0; it.a0 < ce; it.a0 += most) {
+    it.n = ce - it.a0 < most ? ce - it.a0 : most;
+    sl_load(it, smem);
+    sl_columns(it, mx, false, my, false, smem, smem + SL_BUF, [&](int ap, int a, cd val) { dst[ap * ce + a] = val; });
+  }
+  normalise_by_trace(dst, dst, ce, trace_sh);
+}
+
 // A whole sweep in one cooperative launch: node levels in order (the
 // asynchronous schedule's dependency levels), a grid barrier after each, then
-// the edge pass. Every half-edge is computed exactly as bp_node_generic does.
+// the edge pass. Every half-edge is computed exactly as dqz_bp_node_update does:
+// by slices (SLICES) from SL_MIN_CHI, as bp_node_generic below.
+template <bool SLICES>
 __global__ void __launch_bounds__(BP_THREADS) bp_sweep_levels_kernel(
     dqz_graph_t g, const cd *__restrict__ T, const cd *n2e_old, const cd *e2n_old, cd *n2e_new, cd *e2n_new,
     const uint8_t *__restrict__ src_sel, const uint8_t *__restrict__ edge_new, const int32_t *__restrict__ halves,
     const int32_t *__restrict__ level_off, int n_levels, int max_slice, int max_chi, unsigned *sync,
     int *error_flag) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cd *out = reinterpret_cast<cd *>(smem_raw + 48 * sizeof(double));
+  cd *out = reinterpret_cast<cd *>(smem_raw);
   cd *bufA = out + (long long)max_chi * max_chi;
   cd *bufB = bufA + max_slice;
   __shared__ cd trace_sh;
   unsigned gen = 0;
   for (int lv = 0; lv < n_levels; ++lv) {
-    for (int item = level_off[lv] + blockIdx.x; item < level_off[lv + 1]; item += gridDim.x)
-      node_update_half(g, T, n2e_old, e2n_old, n2e_new, src_sel, halves[item], out, bufA, bufB, trace_sh);
+    for (int item = level_off[lv] + blockIdx.x; item < level_off[lv + 1]; item += gridDim.x) {
+      if (SLICES)
+        node_update_half_slices(g, T, n2e_old, e2n_old, n2e_new, src_sel, halves[item], out, max_slice, max_chi,
+                                trace_sh);
+      else
+        node_update_half(g, T, n2e_old, e2n_old, n2e_new, src_sel, halves[item], out, bufA, bufB, trace_sh);
+    }
     if (!grid_barrier(sync, gen, error_flag)) return;
   }
   // edge pass: e2n_new[h] = (edge_new[h] ? n2e_new : n2e_old)[twin(h)], one warp per half-edge
@@ -1118,13 +1157,14 @@ extern "C" int dqz_bp_sweep_levels(const dqz_graph_t *g, const void *tensors, co
   // Small nodes (bond slices up to 256 elements) and narrow levels (at most
   // two half-edges per warp): the whole sweep in one CTA, a warp per
   // half-edge and __syncthreads between levels (no grid barrier). Knob
-  // DQZ_TUNE_SWEEP_ONECTA: 1 = never, 2 = wherever the warps' buffers fit.
+  // DQZ_TUNE_SWEEP_ONECTA: 1 = never, 2 = wherever the warps' buffers fit. From
+  // SL_MIN_CHI only by the knob: its sums are not those of the node update by slices.
   {
     const int knob = dqz_get_tuning(DQZ_TUNE_SWEEP_ONECTA);
     const size_t per_warp = onecta_warp_elems(max_slice, max_chi) * sizeof(cd);
     int warps = (int)(BP_SMEM_LIMIT / per_warp);
     if (warps > ONECTA_THREADS / 32) warps = ONECTA_THREADS / 32;
-    const bool rule = max_slice <= 256 && warps >= 8 && max_level <= 2 * warps;
+    const bool rule = max_chi < SL_MIN_CHI && max_slice <= 256 && warps >= 8 && max_level <= 2 * warps;
     if (knob != 1 && warps >= 1 && (rule || knob == 2)) {
       DQZ_SMEM_ATTR_ONCE(bp_sweep_onecta_kernel, BP_SMEM_LIMIT);
       bp_sweep_onecta_kernel<<<1, 32 * warps, (size_t)warps * per_warp, stream>>>(
@@ -1134,13 +1174,19 @@ extern "C" int dqz_bp_sweep_levels(const dqz_graph_t *g, const void *tensors, co
       return DQZ_OK;
     }
   }
-  const size_t smem = bp_smem_bytes(max_slice, max_chi, false);
+  size_t smem = bp_smem_bytes(max_slice, max_chi, false);
   if (smem > BP_SMEM_LIMIT) return DQZ_ERR_UNSUPPORTED;  // the per-level launches use global scratch then
-  DQZ_SMEM_ATTR_ONCE(bp_sweep_levels_kernel, BP_SMEM_LIMIT);
+  auto *kernel = max_chi >= SL_MIN_CHI ? bp_sweep_levels_kernel<true> : bp_sweep_levels_kernel<false>;
+  if (max_chi >= SL_MIN_CHI) {
+    if (smem < SL_SMEM) smem = SL_SMEM;
+    DQZ_SMEM_ATTR_ONCE(bp_sweep_levels_kernel<true>, BP_SMEM_LIMIT);
+  } else {
+    DQZ_SMEM_ATTR_ONCE(bp_sweep_levels_kernel<false>, BP_SMEM_LIMIT);
+  }
   int dev = 0, sms = 148, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return DQZ_ERR_CUDA;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bp_sweep_levels_kernel, BP_THREADS, smem) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BP_THREADS, smem) !=
           cudaSuccess ||
       per_sm < 1)
     return DQZ_ERR_UNSUPPORTED;
@@ -1157,7 +1203,7 @@ extern "C" int dqz_bp_sweep_levels(const dqz_graph_t *g, const void *tensors, co
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, bp_sweep_levels_kernel, *g, (const cd *)tensors, (const cd *)n2e_old,
+  if (cudaLaunchKernelEx(&cfg, kernel, *g, (const cd *)tensors, (const cd *)n2e_old,
                          (const cd *)e2n_old, (cd *)n2e_new, (cd *)e2n_new, src_sel, edge_new, halves, level_off,
                          (int)n_levels, (int)max_slice, (int)max_chi, (unsigned *)sync, (int *)error_flag) !=
       cudaSuccess)

@@ -186,9 +186,10 @@ int dqz_pack_bf16_umma_nodes(const dqz_graph_t *g, const void *tensors_c64, void
  * memory (use the per-level launches then). Small nodes (slices up to 256
  * elements) with narrow levels run in one CTA instead: a warp per half-edge,
  * a CTA barrier between levels, the same results (knob
- * DQZ_TUNE_SWEEP_ONECTA). For bonds below 8 the messages are those of the
- * per-level launches bit for bit; above, dqz_bp_node_update contracts on the
- * FP64 tensor cores (as dqz_bp_sweep_sliced does) and agrees to rounding. */
+ * DQZ_TUNE_SWEEP_ONECTA) where the bonds are below 8; from 8 on, where
+ * dqz_bp_node_update contracts on the FP64 tensor cores, every half-edge runs
+ * that form here too (the one-CTA form, if the knob asks for it, agrees to
+ * rounding). */
 int dqz_bp_sweep_levels(const dqz_graph_t *g, const void *tensors, const void *n2e_old, const void *e2n_old,
                         void *n2e_new, void *e2n_new, const uint8_t *src_sel, const uint8_t *edge_new,
                         const int32_t *halves, const int32_t *level_off, int32_t n_levels, int32_t max_level,
@@ -204,7 +205,7 @@ int dqz_bp_sweep_levels(const dqz_graph_t *g, const void *tensors, const void *n
  * order its incoming message as offset * 4 + source (DQZ_SRC_*: the offset
  * into e2n_old, n2e_old or n2e_new). A warp per item, a CTA barrier between
  * levels, then the edge pass; the same results as dqz_bp_sweep_levels, bit
- * for bit. DQZ_ERR_UNSUPPORTED when a warp's buffers (two bond slices, the
+ * for bit below bond 8 and to rounding from there. DQZ_ERR_UNSUPPORTED when a warp's buffers (two bond slices, the
  * node tensor, its messages) do not fit in shared memory eight times. */
 #define DQZ_PLAN_WORDS (5 + DQZ_MAX_DEGREE + DQZ_MAX_DEGREE - 1)
 int dqz_bp_sweep_planned(const dqz_graph_t *g, const void *tensors, const void *n2e_old, const void *e2n_old,
