@@ -110,7 +110,7 @@ class GraphLayout:
         return self.edge_chi[self.half_edge]
 
     def _shape(self):
-        """(max bond, max node size, max bond slice, uniform_k3_chi, k3_shape),
+        """(max bond, max node size, max bond slice, uniform_k3_chi, k3_shape, k3_density),
         kept for the bond dimensions they were computed from: a sweep asks for
         them on every call, and small graphs' sweeps last a few microseconds."""
         key = self.edge_chi.tobytes()
@@ -126,7 +126,19 @@ class GraphLayout:
             if k3 and np.all(self.phys == 2) and max_chi in (8, 16) and np.all(self.edge_chi == max_chi):
                 uniform = max_chi
             shape = (max_chi, 1 if uniform else 0) if k3 and max_chi <= 16 else None
-            value = (max_chi, int(sizes.max(initial=1)), max_slice, uniform, shape)
+            # density: a padded node costs pad^3 d^2 however small its bonds, the generic form
+            # follows the bonds and splits nodes above shared memory. Least number of nodes for
+            # the tensor-core form, measured on 3-regular graphs, us, that / generic: 8,190 nodes,
+            # d 2: bond 4 105 / 145, 8 142 / 372, 9 1174 / 513, 11 1224 / 1130, 12 1266 / 1643,
+            # 16 1486 / 3383; d 4: bond 4 267 / 180, 6 298 / 378, 10 2862 / 2405, 12 3165 /
+            # 3766; 16 nodes, d 4: bond 12 60 / 54, 16 78 / 50; d 8: bond 6 53 / 34; 100 nodes,
+            # d 4: bond 12 61 / 62, 16 79 / 98.
+            density = None
+            if shape:
+                d_max, pad = int(self.phys.max()), 8 if max_chi <= 8 else 16
+                if (d_max <= 2 and pad == 8) or float((sizes / self.phys).mean()) >= 0.4 * pad**3:
+                    density = 0 if d_max <= 3 else 38
+            value = (max_chi, int(sizes.max(initial=1)), max_slice, uniform, shape, density)
             self._shape_kept = (key, value)
         return value
 
@@ -141,6 +153,12 @@ class GraphLayout:
         tensor-core kernels cover every node (degree 3, bonds up to 16, zero-
         padded to 8 or 16 when not uniform); None otherwise."""
         return self._shape()[4]
+
+    def k3_density(self, n_nodes: int) -> bool:
+        """Whether the degree-3 tensor-core kernel is the faster one for the
+        densities of ``n_nodes`` nodes."""
+        least = self._shape()[5]
+        return least is not None and n_nodes >= least
 
     # ------------------------------------------------------------ offsets
     def _finish(self):

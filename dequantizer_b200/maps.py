@@ -562,9 +562,8 @@ def density_packed(layout: GraphLayout, T, e2n, nodes: List[int]) -> torch.Tenso
     idx = torch.tensor(nodes, dtype=torch.int32, device=dev)
     mp = _lib.MAX_PHYS
     rho = torch.zeros((len(nodes), mp * mp), dtype=torch.complex128, device=dev)
-    k3 = layout.k3_shape()
-    if k3:
-        _lib.call("dqz_density_k3", layout.gptr, *k3, T.data_ptr(), e2n.data_ptr(), idx.data_ptr(), len(nodes),
+    if layout.k3_density(len(nodes)):
+        _lib.call("dqz_density_k3", layout.gptr, *layout.k3_shape(), T.data_ptr(), e2n.data_ptr(), idx.data_ptr(), len(nodes),
                   rho.data_ptr(), error_flag(dev).data_ptr(), _lib.stream_handle())
         d = int(layout.phys[nodes[0]]) if nodes else 2
         return rho[:, : d * d].reshape(len(nodes), d, d)
