@@ -154,9 +154,10 @@ __global__ void __launch_bounds__(BP_THREADS) bp_node_generic(dqz_graph_t g, con
 
 // Bonds from SL_MIN_CHI: the node update by blocks of slices on the FP64 tensor
 // cores (bp_slices.cuh), block blockIdx.y of half-edge halves[blockIdx.x], columns
-// left unnormalised for bp_trace_kernel. Nodes outside that form's shapes run the
-// generic update in their first block's CTA (two slices in shared memory). Below
-// the bound the one-launch sweeps of small nodes are faster, and must agree with
+// left unnormalised for bp_trace_kernel. Nodes outside that form's shapes share the
+// generic update's columns out among the same CTAs (two slices in shared memory):
+// 4-regular graph of 200 nodes, bond 8, 378 us (400 by one CTA a half-edge here, 382
+// by the generic kernel alone); 26 nodes 73 us (113, 102). Below the bound the one-launch sweeps of small nodes are faster, and must agree with
 // this entry bit for bit.
 constexpr int SL_MIN_CHI = 8;
 
@@ -189,9 +190,8 @@ __global__ void __launch_bounds__(SL_THREADS, 2) bp_node_slices(dqz_graph_t g, c
     sl_columns(it, mx, false, my, false, buf, buf + SL_BUF, [&](int ap, int a, cd val) { dst[ap * ce + a] = val; });
     return;
   }
-  if (blockIdx.y) return;
   const int ce = s.dims[e];
-  for (int a = 0; a < ce; ++a)
+  for (int a = blockIdx.y; a < ce; a += gridDim.y)
     node_slice_column(g, Tv, s, e, n2e_old, e2n_old, n2e_new, src_sel, a, buf, buf + max_slice,
                       [&](int ap, cd val) { dst[ap * ce + a] = val; });
 }
