@@ -1228,16 +1228,21 @@ extern "C" int dqz_density_matrices(const dqz_graph_t *g, const void *tensors, c
   const bool use_scratch = need > SMEM_LIMIT;
   if (use_scratch && !scratch) return DQZ_ERR_ARG;
   DQZ_SMEM_ATTR_ONCE(density_kernel, SMEM_LIMIT);
-  if (!use_scratch) {
-    density_kernel<<<n_nodes, GAUGE_THREADS, need, stream>>>(*g, (const cd *)tensors, (const cd *)e2n, nodes, n_nodes,
-                                                            (cd *)rho, max_size, nullptr, 0);
+  // Nodes within shared memory keep the whole-node form: one launch, and no pass over T
+  // per block. So do graphs of mean degree above 3: their largest nodes are outside the
+  // slices' form, whose launches would only add to theirs (4-regular graph of 200 nodes,
+  // bond 8, us: 181, 197 with them; 10 x 10 lattice 155, 163).
+  if (!use_scratch || g->n_halves > 3ll * g->n_nodes) {
+    const int grid = use_scratch && n_nodes > SCRATCH_GRID ? SCRATCH_GRID : n_nodes;
+    density_kernel<<<grid, GAUGE_THREADS, use_scratch ? 0 : need, stream>>>(
+        *g, (const cd *)tensors, (const cd *)e2n, nodes, n_nodes, (cd *)rho, max_size,
+        use_scratch ? (cd *)scratch : nullptr, 0);
     DQZ_CHECK_LAUNCH();
     return DQZ_OK;
   }
   // Above shared memory: blocks of slices, then the nodes outside that form one CTA
   // each. The blocks' shares (a slot of DENS_BLOCKS x DENS_PP per node) take less of
-  // the scratch than the node slices they are followed by. Nodes within shared memory
-  // keep the whole-node form: one launch, and no pass over T per block.
+  // the scratch than the node slices they are followed by.
   static_assert((size_t)DENS_BLOCKS * DENS_PP * sizeof(cd) <= SMEM_LIMIT, "the shares fit a node's scratch");
   DQZ_SMEM_ATTR_ONCE(density_slices_kernel, SMEM_LIMIT);
   for (int first = 0; first < n_nodes; first += SCRATCH_GRID) {
