@@ -750,9 +750,30 @@ extern "C" size_t dqz_simple_update_scratch_bytes(int32_t n, int32_t max_rows, i
   return su_marks_bytes(n) + (one_cta > cluster ? one_cta : cluster);
 }
 
+// Whether the register form goes first. It ends a job sooner (both sides and the core
+// on CTAs of their own), but takes three CTAs a job where the one-CTA kernel runs
+// several jobs per SM, so the smaller the matrices and the larger the batch, the
+// better the latter. Measured between degree-3 nodes, d 2, us, register form / one-CTA
+// kernel (from 256 rows the forms that follow): gate rank 2, bond 3 29 jobs 87 / 85;
+// bond 4 56 99 / 110, 114 131 / 111; bond 5 56 124 / 150, 114 164 / 155; bond 7 114 216 /
+// 236, 223 315 / 290; bond 8 449 631 / 715, 750 1001 / 904; bond 9 (above 64 rows of
+// other bonds a column takes four times the registers) 114 339 / 420, 223 533 / 490; bond
+// 10 449 1096 / 1238, 750 1810 / 1484; bond 11 1405 3417 / 4166; bond 16 1405 5262 /
+// 12469; rank 1, bond 8 56 110 / 136, 114 158 / 137; bond 10 56 174 /
+// 217, 114 265 / 219; bond 12 1405 2800 / 3629.
+static bool su_reg_first(int n, int max_rows, int max_cols) {
+  if (max_rows >= SUF_MIN_ROWS || max_cols >= 22) return true;
+  if (max_cols >= 20) return n <= 512;
+  if (max_cols >= 16 && max_rows <= 128) return n <= 512;
+  if (max_cols >= 14) return n <= 180;
+  if (max_cols >= 10) return n <= 80;
+  return max_cols >= 7 && n <= 64;
+}
+
 extern "C" size_t dqz_simple_update_workspace_bytes(int32_t n, int32_t max_rows, int32_t max_cols) {
   const size_t least = dqz_simple_update_scratch_bytes(n, max_rows, max_cols);
-  const size_t reg = n > 0 ? su_marks_bytes(n) + su_reg_scratch_bytes(n, max_rows) : 0;
+  const size_t reg =
+      n > 0 && su_reg_first(n, max_rows, max_cols) ? su_marks_bytes(n) + su_reg_scratch_bytes(n, max_rows) : 0;
   return least > reg ? least : reg;
 }
 
@@ -787,14 +808,13 @@ extern "C" int dqz_simple_update_ws(const dqz_graph_t *g, void *tensors, double 
   // 2 = the cluster forms at any batch size, 3 = no global-workspace form.
   const int knob = dqz_get_tuning(DQZ_TUNE_SU_ONCHIP);
   // jobs whose factors fit the registers (bonds up to 16 between degree-3 nodes)
-  // first, whatever the batch size; the forms below take the jobs it left. Measured
-  // at bond 16, ms for a layer of gates: 60 gates (levels of 1 to 11) 3.5 here, 6.7 on
+  // first; the forms below take the jobs it left. Measured at bond 16, ms for a layer of gates: 60 gates (levels of 1 to 11) 3.5 here, 6.7 on
   // the cluster forms, 20 on the one-CTA kernel; 3,600 gates 16.4, 34.9, 55.9.
   // A workspace that holds one job's factors is enough: it sets how many jobs are in
   // flight; one that does not (small bonds, the least scratch) leaves all to the others.
   int chained = 0;
   const size_t room = scratch_bytes - su_marks_bytes(n);
-  if (knob == 0 && room >= su_reg_scratch_bytes(1, max_rows)) {
+  if (knob == 0 && su_reg_first(n, max_rows, max_cols) && room >= su_reg_scratch_bytes(1, max_rows)) {
     marks = static_cast<uint8_t *>(scratch);
     const int st = su_reg(g, tensors, lambdas, edges, ctrl_is_first, halves, ranks, n, eps, max_rank, max_rows, err,
                           entropy, marks, job_scratch, room, stream);
@@ -915,7 +935,7 @@ extern "C" int dqz_simple_update_noalloc(const dqz_graph_t *g, void *tensors, do
   uint8_t *marks = nullptr;
   size_t room = (size_t)DQZ_NOALLOC_SCRATCH_BYTES;
   const size_t mb = su_marks_bytes(n), one = su_reg_scratch_bytes(1, max_rows);
-  if (dqz_get_tuning(DQZ_TUNE_SU_ONCHIP) == 0 && mb + (per_job > one ? per_job : one) <= room &&
+  if (dqz_get_tuning(DQZ_TUNE_SU_ONCHIP) == 0 && su_reg_first(n, max_rows, max_cols) && mb + (per_job > one ? per_job : one) <= room &&
       mb + one <= dqz_simple_update_scratch_bytes(n, max_rows, max_cols)) {
     marks = static_cast<uint8_t *>(scratch);
     scratch = static_cast<char *>(scratch) + mb;

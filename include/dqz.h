@@ -422,10 +422,10 @@ size_t dqz_simple_update_scratch_bytes(int32_t n, int32_t max_rows, int32_t max_
 
 /* The same with a scratch of a stated size, at least
  * dqz_simple_update_scratch_bytes. Jobs whose factors fit the registers (bonds up
- * to 16 between degree-3 nodes) run a register-resident form before the others,
- * as many at a time as the scratch holds workspace slices (none: the forms above
- * take them); dqz_simple_update_workspace_bytes holds them all, up to four per
- * SM. */
+ * to 16 between degree-3 nodes) run a register-resident form before the others
+ * where it is the faster for max_rows, max_cols and n, as many at a time as the
+ * scratch holds workspace slices (none: the forms above take them);
+ * dqz_simple_update_workspace_bytes holds them all, up to four per SM. */
 int dqz_simple_update_ws(const dqz_graph_t *g, void *tensors, double *lambdas, const int32_t *edges,
                          const uint8_t *ctrl_is_first, const void *halves, const int32_t *ranks, int32_t n,
                          double eps, int32_t max_rank, int32_t max_rows, int32_t max_cols, double *err,
