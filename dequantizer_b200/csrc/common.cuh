@@ -38,9 +38,12 @@ __device__ __forceinline__ void cfmac(cd &acc, cd a, cd b) {
   acc.y = fma(a.x, b.y, acc.y);
   acc.y = fma(-a.y, b.x, acc.y);
 }
+// The fused steps are spelled out: which product of a sum the compiler fuses may differ
+// from kernel to kernel, and kernels that divide the same message by the same trace
+// have to agree bit for bit.
 __device__ __forceinline__ cd cdiv(cd a, cd b) {
-  double den = b.x * b.x + b.y * b.y;
-  return mk((a.x * b.x + a.y * b.y) / den, (a.y * b.x - a.x * b.y) / den);
+  const double den = fma(b.x, b.x, __dmul_rn(b.y, b.y));
+  return mk(fma(a.x, b.x, __dmul_rn(a.y, b.y)) / den, fma(a.y, b.x, -__dmul_rn(a.x, b.y)) / den);
 }
 
 // ------------------------------------------------- reciprocals and roots
