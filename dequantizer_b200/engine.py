@@ -34,7 +34,8 @@ import torch
 from . import _lib
 from .graph import TensorGraph
 from .layout import GraphLayout
-from .maps import BF16_KERNELS, Topology, bp_sweep, density_packed, error_flag, vidal_distance_packed, vidal_gauge_packed
+from .maps import (BF16_KERNELS, SLICED_MIN_CHI, Topology, bp_sweep, density_packed, error_flag, vidal_distance_packed,
+                   vidal_gauge_packed)
 
 log = logging.getLogger(__name__)
 
@@ -289,8 +290,12 @@ class BPEngine:
         if self.precision == "fp64":
             if self.layout.uniform_k3_chi() or (self.layout.k3_shape() and len(self.topo.levels) == 1):
                 return len(self.topo.levels)  # the edge pass runs in the node update's launch (dqz_bp_sweep_k3)
-            if len(self.topo.levels) > 1:
-                return 1  # every level and the edge pass in one cooperative launch (dqz_bp_sweep_levels)
+            L, widest = self.layout, max(len(lv) for lv in self.topo.levels)
+            on_chip = _lib.lib().dqz_bp_node_scratch_bytes(widest, L.max_slice(), L.max_chi()) == 0
+            if len(self.topo.levels) > 1 and on_chip:
+                return 1  # every level and the edge pass in one launch (dqz_bp_sweep_levels and its forms)
+            if on_chip and L.max_chi() >= SLICED_MIN_CHI:
+                return 2 * len(self.topo.levels) + 1  # dqz_bp_node_update by slices: columns, then traces
         if self.precision == "fp32":
             return len(self.topo.levels)  # likewise (dqz_bp_sweep_k3_c64)
         return len(self.topo.levels) + 1
