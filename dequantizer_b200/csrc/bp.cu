@@ -660,12 +660,12 @@ __global__ void __launch_bounds__(PLAN_THREADS) bp_sweep_whole_kernel(
         const int after = f + 1 == e ? f + 2 : f + 1;
         const int4 nb = W.bond[after < k ? after : e];  // on its way during the product; the pairs' at the end
         const cd *m = Ms + W.moff[f];
-      switch (bond.y) {
-        case 2: plan_fibers<2, 2>(bond, size, cur, nxt, m); break;
-        case 3: plan_fibers<3, 2>(bond, size, cur, nxt, m); break;
-        case 4: plan_fibers<4, 1>(bond, size, cur, nxt, m); break;
-        default: plan_product<4>(bond, size, cur, nxt, m);
-      }
+        switch (bond.y) {
+          case 2: plan_fibers<2, 2>(bond, size, cur, nxt, m); break;
+          case 3: plan_fibers<3, 2>(bond, size, cur, nxt, m); break;
+          case 4: plan_fibers<4, 1>(bond, size, cur, nxt, m); break;
+          default: plan_product<4>(bond, size, cur, nxt, m);
+        }
         bond = nb;
         f = after;
         __syncwarp();

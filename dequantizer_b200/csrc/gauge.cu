@@ -644,8 +644,9 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_distance_kernel(dqz_graph
       if (Rm[i * ce + i].x > eps) Rm[i * ce + i].x -= idv;
     __syncthreads();
     // the trace norm from the eigenvalues (tridiagonal reduction, then counts or,
-    // above bond 32, implicit QL; the staging area is free again for its vectors).
-    // Measured at 288 half-edges of bond 32: 672 us with QL, 504 us with counts (R on
+    // above bond 32, the shared-memory form with bisection; the staging area is free again
+    // for its vectors). Measured at 288 half-edges of bond 32: 672 us with that form, whose
+    // reduction takes five CTA barriers a column, 504 us with two warps' registers (R on
     // the FP64 tensor cores, one CTA per SM for its registers: 523 us).
     const double t = ce <= 32 ? cta_trace_norm32(Rm, ce, ce, *reinterpret_cast<TraceNorm32Smem *>(U))
                               : herm_trace_norm(Rm, ce, ce, U, U + DQZ_MAX_CHI,

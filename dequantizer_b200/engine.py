@@ -273,7 +273,8 @@ class BPEngine:
     def sweep(self, mid_event=None) -> None:
         """One BP sweep; the previous message set is kept for ``distance``.
         ``mid_event`` (a torch.cuda.Event) is recorded between the node
-        updates and the edge pass, to time the node-update kernel alone."""
+        updates and the edge pass, to time the node-update kernel alone, or after
+        both where one launch does both (bp_sweep)."""
         n2e_new, e2n_new = self._spare
         if self.T_bf16 is not None and self._bf16_stale:
             pack = "dqz_pack_bf16_umma" if self.bf16_kernel == "tcgen05" else "dqz_pack_bf16_planes"

@@ -163,11 +163,12 @@ class Topology:
             he = layout.half_edge
             ce = np.where(he >= 0, layout.edge_chi[np.maximum(he, 0)], 0).astype(np.int64)
             size = layout.node_sizes()[layout.half_node] // np.maximum(ce, 1)  # entries of a slice
+            sms = torch.cuda.get_device_properties(device).multi_processor_count
             halves, slices, off = [], [], [0]
             for lv in self.levels:
                 c, sz = ce[lv], size[lv]
                 elems = SLICE_BLOCK_ELEMS
-                while elems > 256 and int(np.ceil(c / np.maximum(elems // np.maximum(sz, 1), 1)).sum()) < SLICE_SMS:
+                while elems > 256 and int(np.ceil(c / np.maximum(elems // np.maximum(sz, 1), 1)).sum()) < sms:
                     elems //= 2
                 n = np.maximum(elems // np.maximum(sz, 1), 1)
                 cnt = np.where(c > 0, -(-c // n), 0)
@@ -266,13 +267,13 @@ BF16_KERNELS = {"tcgen05": "dqz_bp_node_update_k3_umma", "mma_sync": "dqz_bp_nod
 # has a handful of half-edges of ~50 MFLOP each
 SLICED_MIN_CHI = 8
 SLICE_BLOCK_ELEMS = 4096  # entries of a block of slices (bp_slices.cuh)
-SLICE_SMS = 148
 
 
 def bp_sweep(layout: GraphLayout, topo: Topology, T, n2e_old, e2n_old, n2e_new, e2n_new, mid_event=None,
              T_bf16=None, bf16_kernel: str = "tcgen05"):
-    """One sweep on packed arenas: node updates level by level, then the edge pass
-    (``mid_event``, a torch.cuda.Event, is recorded between the two).
+    """One sweep on packed arenas: node updates level by level, then the edge pass.
+    ``mid_event``, a torch.cuda.Event, is recorded between the two, or after both
+    where one launch does both (all but the BF16 forms and the generic one).
 
     complex128 arenas use the degree-3 tensor-core kernel where it covers
     every node (layout.k3_shape), the generic kernels otherwise;
