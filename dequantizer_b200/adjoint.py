@@ -58,6 +58,12 @@ class FixedPointProblem:
         # shapes of the tensor-core kernels (bp_k3.cu, adjoint_k3.cu): messages
         # read at the node's own half-edges, and the change of an iteration
         self._k3 = L.k3_shape()
+        # a padded node's adjoint costs as many slabs as it has physical indices, the generic
+        # form follows the bonds (random 3-regular graphs, a transposed sweep / with the tensor
+        # cotangent, us, tensor-core form against generic: 8,190 nodes, d 8, bond 2 1387 / 2388
+        # against 975 / 1270, bond 3 1388 / 2394 against 1275 / 1568, bond 4 1393 / 2418 against
+        # 1869 / 2382; d 4, bond 2 726 / 1231 against 973 / 1260)
+        self._k3_vjp = None if self._k3 and L.max_chi() <= 3 and int(L.phys.max()) >= 6 else self._k3
         self._own = torch.zeros(max(L.n_halves, 1), dtype=torch.uint8, device=L.device)
         self.last_sweeps = 0
         self.last_adjoint_sweeps = 0
@@ -107,7 +113,7 @@ class FixedPointProblem:
         """Transposed node update: returns the e2n cotangent arena; adds the
         node-tensor cotangent into t_cot when given."""
         L = self.layout
-        if self._k3:
+        if self._k3_vjp:
             out = torch.zeros_like(e2n)
             self._vjp_k3(T, e2n, n2e_cot, self._raw_messages(T, e2n), out, t_cot=t_cot)
             return out
@@ -140,11 +146,11 @@ class FixedPointProblem:
         change is <= tol * max|g|; adds the tensor cotangent of x into t_cot."""
         scale = float(g.abs().max()) or 1.0
         change = torch.zeros(1, dtype=torch.float64, device=g.device)
-        raw = self._raw_messages(T, e2n) if self._k3 else None  # the same in every transposed sweep
+        raw = self._raw_messages(T, e2n) if self._k3_vjp else None  # the same in every transposed sweep
         x = g.clone()
         it = 0
         for it in range(1, max_sweeps + 1):
-            if self._k3:
+            if self._k3_vjp:
                 x_new = torch.empty_like(x)
                 change.zero_()
                 self._vjp_k3(T, e2n, x, raw, x_new, add=g, change=change)
@@ -156,7 +162,7 @@ class FixedPointProblem:
             if d <= tol * scale:
                 break
         self.last_adjoint_sweeps = it
-        if self._k3:
+        if self._k3_vjp:
             self._vjp_k3(T, e2n, x, raw, None, t_cot=t_cot)
         else:
             self.node_vjp(T, e2n, x, t_cot)
