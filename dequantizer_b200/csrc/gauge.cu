@@ -797,7 +797,9 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_distance_warp_kernel(
 // Memory-bound: the square roots of the lambdas are taken once per node, not per
 // entry, and positions are 32-bit. Measured over the 21 calls of a kicked-Ising run
 // on the 127-qubit heavy-hex lattice (bonds growing to 32): 2.10 ms before, 0.57 ms
-// (0.64 ms with 1,024 threads a node).
+// (0.64 ms with 1,024 threads a node). More than two nodes per SM: half the threads, so
+// that twice as many are resident (3-regular graphs, us, 512 / 256 threads: 200 nodes bond
+// 16 43 / 56; 300 nodes 68 / 64; 3,000 nodes bond 2 50 / 29, bond 8 101 / 75).
 constexpr int SYM_THREADS = 512;
 __global__ void __launch_bounds__(SYM_THREADS) symmetric_kernel(dqz_graph_t g, const cd *__restrict__ Tin,
                                                                 const double *__restrict__ lambdas, double eps,
@@ -1196,8 +1198,8 @@ extern "C" int dqz_symmetric_gauge(const dqz_graph_t *g, const void *tensors_in,
                                    void *tensors_out, cudaStream_t stream) {
   if (!g || !tensors_in || !lambdas || !tensors_out) return DQZ_ERR_ARG;
   if (g->n_nodes == 0) return DQZ_OK;
-  symmetric_kernel<<<g->n_nodes, SYM_THREADS, 0, stream>>>(*g, (const cd *)tensors_in, lambdas, eps,
-                                                              (cd *)tensors_out);
+  symmetric_kernel<<<g->n_nodes, g->n_nodes > 2 * SM_COUNT ? SYM_THREADS / 2 : SYM_THREADS, 0, stream>>>(
+      *g, (const cd *)tensors_in, lambdas, eps, (cd *)tensors_out);
   DQZ_CHECK_LAUNCH();
   return DQZ_OK;
 }
