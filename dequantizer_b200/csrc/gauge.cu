@@ -28,7 +28,7 @@ constexpr size_t WARP_BLOCK_SMEM = 96 * 1024;
 constexpr int SM_COUNT = 148;
 constexpr int SCRATCH_GRID = SM_COUNT * 4;
 
-// Left to another kernel (edges: in lambda[0]; nodes: in rho[0]).
+// An edge left to another kernel (in lambda[0]).
 __device__ __forceinline__ bool is_marked(double x) { return __double_as_longlong(x) == (long long)ES_MARK; }
 
 // ----------------------------------------------------------- vidal edges
@@ -869,8 +869,54 @@ __global__ void lambdas_to_messages_kernel(dqz_graph_t g, const double *__restri
 }
 
 // -------------------------------------------------------- density matrices
-// Nodes of degree up to 3 with bonds up to 32 whose tensor is above shared memory:
-// block blockIdx.y of the slices of the first bond, one CTA. Slices a' of
+// rho of one node (into out) by the whole CTA, the mode products in bufA / bufB (the node's size each). Ends with
+// a barrier.
+__device__ __forceinline__ void density_node(const dqz_graph_t &g, const cd *__restrict__ Tall,
+                                             const cd *__restrict__ e2n, int v, cd *out, cd *bufA, cd *bufB) {
+  __shared__ cd rho_sh[DQZ_MAX_PHYS * DQZ_MAX_PHYS];
+  __shared__ cd trace_sh;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  NodeShape s;
+  load_shape(g, v, s);
+  const cd *T = Tall + g.node_off[v];
+  for (long long i = threadIdx.x; i < s.size; i += blockDim.x) bufA[i] = T[i];
+  __syncthreads();
+  cd *cur = bufA, *nxt = bufB;
+  long long L = 1;
+  for (int f = 0; f < s.k; ++f) {
+    const int q = s.dims[f];
+    const long long R = s.size / L / q;
+    const cd *m = e2n + g.half_msg_off[s.half0 + f];
+    mode_product<false>(cur, nxt, L, q, q, R, m, q, 1);
+    __syncthreads();
+    cd *t = cur;
+    cur = nxt;
+    nxt = t;
+    L *= q;
+  }
+  const int d = s.d;
+  const long long B = s.size / d;
+  for (int p = warp; p < d * d; p += nw) {
+    const int si = p / d, sj = p % d;
+    cd acc = czero();
+    for (long long b = lane; b < B; b += 32) cfmac(acc, T[b * d + sj], cur[b * d + si]);
+    acc = warp_csum(acc);
+    if (lane == 0) rho_sh[si * d + sj] = acc;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    cd tr = czero();
+    for (int i = 0; i < d; ++i) tr = cadd(tr, rho_sh[i * d + i]);
+    trace_sh = tr;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < d * d; i += blockDim.x) out[i] = cdiv(rho_sh[i], trace_sh);
+  __syncthreads();
+}
+
+// Nodes of degree up to 3 with bonds up to 32 in graphs with tensors above shared memory:
+// block blockIdx.y of the slices of the first bond, one CTA (the other nodes: the whole
+// node in the first block's CTA, as density_kernel). Slices a' of
 // m_0 T are summed over a from T (read through L2 once per block, whole rows), the
 // other bonds' messages applied in shared memory (bp_slices.cuh), and the block's
 // share of rho summed in a fixed order; density_finish adds the blocks in order.
@@ -884,7 +930,8 @@ constexpr int DENS_GRID = 16;        // blocks in flight per node (the others fo
 __global__ void __launch_bounds__(SL_THREADS, 2) density_slices_kernel(dqz_graph_t g, const cd *__restrict__ Tall,
                                                                        const cd *__restrict__ e2n,
                                                                        const int32_t *__restrict__ nodes, cd *rho,
-                                                                       cd *part) {
+                                                                       cd *scratch, int max_size) {
+  static_assert(SL_THREADS == GAUGE_THREADS, "both forms in one launch");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cd *buf = reinterpret_cast<cd *>(smem_raw), *sM = buf + SL_BUF;
   __shared__ cd sums[SL_THREADS / 32];
@@ -893,8 +940,10 @@ __global__ void __launch_bounds__(SL_THREADS, 2) density_slices_kernel(dqz_graph
   NodeShape s;
   load_shape(g, v, s);
   SliceItem it;
+  cd *part = scratch + (long long)item * 2 * max_size;  // the node's shares, or its mode products
   if (!sl_geometry(s, 0, it.g)) {
-    if (blockIdx.y == 0 && tid == 0) rho[(long long)item * DENS_PP].x = __longlong_as_double((long long)ES_MARK);
+    if (blockIdx.y == 0)
+      density_node(g, Tall, e2n, v, rho + (long long)item * DENS_PP, part, part + max_size);
     return;
   }
   const int most = sl_count(it.g), ce = it.g.ce, d = s.d;
@@ -945,7 +994,7 @@ __global__ void __launch_bounds__(SL_THREADS, 2) density_slices_kernel(dqz_graph
     const int pairs = d * d, group = pairs >= NW ? 1 : NW / pairs, per = NW / group;
     const unsigned B = (unsigned)it.n * (P / (unsigned)d);
     const FastDiv fB(P / (unsigned)d);
-    cd *out = part + ((long long)item * DENS_BLOCKS + blk) * DENS_PP;
+    cd *out = part + blk * DENS_PP;
     for (int p0 = 0; p0 < pairs; p0 += per) {
       const int p = p0 + w / group, si = p / d, sj = p % d;
       cd acc = czero();
@@ -971,7 +1020,8 @@ __global__ void __launch_bounds__(SL_THREADS, 2) density_slices_kernel(dqz_graph
 
 // rho of the nodes above: the blocks' shares added in order, over the trace.
 __global__ void __launch_bounds__(DENS_PP) density_finish_kernel(dqz_graph_t g, const int32_t *__restrict__ nodes,
-                                                                 cd *rho, const cd *__restrict__ part) {
+                                                                 cd *rho, const cd *__restrict__ scratch,
+                                                                 int max_size) {
   __shared__ cd sh[DENS_PP];
   const int item = blockIdx.x, v = nodes[item], p = threadIdx.x;
   NodeShape s;
@@ -979,9 +1029,10 @@ __global__ void __launch_bounds__(DENS_PP) density_finish_kernel(dqz_graph_t g, 
   SliceGeom geom;
   if (!sl_geometry(s, 0, geom)) return;
   const int d = s.d, most = sl_count(geom), blocks = (geom.ce + most - 1) / most;
+  const cd *part = scratch + (long long)item * 2 * max_size;
   cd t = czero();
   if (p < d * d)
-    for (int b = 0; b < blocks; ++b) t = cadd(t, part[((long long)item * DENS_BLOCKS + b) * DENS_PP + p]);
+    for (int b = 0; b < blocks; ++b) t = cadd(t, part[b * DENS_PP + p]);
   sh[p] = t;
   __syncthreads();
   cd tr = czero();
@@ -992,55 +1043,12 @@ __global__ void __launch_bounds__(DENS_PP) density_finish_kernel(dqz_graph_t g, 
 __global__ void __launch_bounds__(GAUGE_THREADS) density_kernel(dqz_graph_t g, const cd *__restrict__ Tall,
                                                                  const cd *__restrict__ e2n,
                                                                  const int32_t *__restrict__ nodes, int n_nodes,
-                                                                 cd *rho, int max_size, cd *scratch,
-                                                                 int only_marked) {
+                                                                 cd *rho, int max_size, cd *scratch) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cd *bufA = scratch ? scratch + (long long)blockIdx.x * 2 * max_size : reinterpret_cast<cd *>(smem_raw);
-  cd *bufB = bufA + max_size;
-  __shared__ cd rho_sh[DQZ_MAX_PHYS * DQZ_MAX_PHYS];
-  __shared__ cd trace_sh;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int item = blockIdx.x; item < n_nodes; item += gridDim.x) {
-    if (only_marked && !is_marked(rho[(long long)item * DQZ_MAX_PHYS * DQZ_MAX_PHYS].x)) continue;
-    const int v = nodes[item];
-    NodeShape s;
-    load_shape(g, v, s);
-    const cd *T = Tall + g.node_off[v];
-    for (long long i = threadIdx.x; i < s.size; i += blockDim.x) bufA[i] = T[i];
-    __syncthreads();
-    cd *cur = bufA, *nxt = bufB;
-    long long L = 1;
-    for (int f = 0; f < s.k; ++f) {
-      const int q = s.dims[f];
-      const long long R = s.size / L / q;
-      const cd *m = e2n + g.half_msg_off[s.half0 + f];
-      mode_product<false>(cur, nxt, L, q, q, R, m, q, 1);
-      __syncthreads();
-      cd *t = cur;
-      cur = nxt;
-      nxt = t;
-      L *= q;
-    }
-    const int d = s.d;
-    const long long B = s.size / d;
-    for (int p = warp; p < d * d; p += nw) {
-      const int si = p / d, sj = p % d;
-      cd acc = czero();
-      for (long long b = lane; b < B; b += 32) cfmac(acc, T[b * d + sj], cur[b * d + si]);
-      acc = warp_csum(acc);
-      if (lane == 0) rho_sh[si * d + sj] = acc;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      cd tr = czero();
-      for (int i = 0; i < d; ++i) tr = cadd(tr, rho_sh[i * d + i]);
-      trace_sh = tr;
-    }
-    __syncthreads();
-    cd *out = rho + (long long)item * DQZ_MAX_PHYS * DQZ_MAX_PHYS;
-    for (int i = threadIdx.x; i < d * d; i += blockDim.x) out[i] = cdiv(rho_sh[i], trace_sh);
-    __syncthreads();
-  }
+  for (int item = blockIdx.x; item < n_nodes; item += gridDim.x)
+    density_node(g, Tall, e2n, nodes[item], rho + (long long)item * DQZ_MAX_PHYS * DQZ_MAX_PHYS, bufA,
+                 bufA + max_size);
 }
 
 size_t eigh_smem(int max_chi) {
@@ -1239,25 +1247,21 @@ extern "C" int dqz_density_matrices(const dqz_graph_t *g, const void *tensors, c
     const int grid = use_scratch && n_nodes > SCRATCH_GRID ? SCRATCH_GRID : n_nodes;
     density_kernel<<<grid, GAUGE_THREADS, use_scratch ? 0 : need, stream>>>(
         *g, (const cd *)tensors, (const cd *)e2n, nodes, n_nodes, (cd *)rho, max_size,
-        use_scratch ? (cd *)scratch : nullptr, 0);
+        use_scratch ? (cd *)scratch : nullptr);
     DQZ_CHECK_LAUNCH();
     return DQZ_OK;
   }
-  // Above shared memory: blocks of slices, then the nodes outside that form one CTA
-  // each. The blocks' shares (a slot of DENS_BLOCKS x DENS_PP per node) take less of
-  // the scratch than the node slices they are followed by.
+  // Above shared memory: blocks of slices (the blocks' shares, DENS_BLOCKS x DENS_PP, in
+  // the node's own slice of the scratch), the nodes outside that form a CTA each.
   static_assert((size_t)DENS_BLOCKS * DENS_PP * sizeof(cd) <= SMEM_LIMIT, "the shares fit a node's scratch");
   DQZ_SMEM_ATTR_ONCE(density_slices_kernel, SMEM_LIMIT);
   for (int first = 0; first < n_nodes; first += SCRATCH_GRID) {
     const int n = n_nodes - first < SCRATCH_GRID ? n_nodes - first : SCRATCH_GRID;
     cd *out = (cd *)rho + (long long)first * DENS_PP;
     density_slices_kernel<<<dim3(n, DENS_GRID), SL_THREADS, SL_SMEM, stream>>>(
-        *g, (const cd *)tensors, (const cd *)e2n, nodes + first, out, (cd *)scratch);
+        *g, (const cd *)tensors, (const cd *)e2n, nodes + first, out, (cd *)scratch, max_size);
     DQZ_CHECK_LAUNCH();
-    density_finish_kernel<<<n, DENS_PP, 0, stream>>>(*g, nodes + first, out, (const cd *)scratch);
-    DQZ_CHECK_LAUNCH();
-    density_kernel<<<n, GAUGE_THREADS, 0, stream>>>(*g, (const cd *)tensors, (const cd *)e2n, nodes + first, n, out,
-                                                    max_size, (cd *)scratch, 1);
+    density_finish_kernel<<<n, DENS_PP, 0, stream>>>(*g, nodes + first, out, (const cd *)scratch, max_size);
     DQZ_CHECK_LAUNCH();
   }
   return DQZ_OK;
