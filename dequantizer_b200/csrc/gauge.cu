@@ -195,8 +195,9 @@ __device__ __forceinline__ void cta_edge(const dqz_graph_t &g, EdgeCtaSmem &S, i
 
 // Every edge (WARP_MAX_CHI < max_chi <= RJ_MAX); the few it leaves run the first
 // kernel above. Bound by the Jacobi rounds' latency (31 of about 1,200 cycles a
-// sweep, two iterations after another). Measured at 144 edges of bond 32: 768 us,
-// 3,433 us with two-sided rotations and C formed in the original basis.
+// sweep, two iterations after another). Measured at 144 edges of bond 32: 539 us, 1,493
+// us with two-sided rotations and C formed in the original basis; two of them rank-
+// deficient 592 and 2,374 us.
 __global__ void __launch_bounds__(EC_THREADS) vidal_edges_cta_kernel(dqz_graph_t g, const cd *__restrict__ n2e,
                                                                      double eps, cd *orth, double *lambdas, int max_chi,
                                                                      const int32_t *__restrict__ sel, int total) {
