@@ -66,9 +66,8 @@ __device__ __forceinline__ bool sl_geometry(const NodeShape &s, int e, SliceGeom
 
 // Slices that fit a block of this geometry.
 __device__ __forceinline__ int sl_count(const SliceGeom &g) {
-  int n = sl_block(g.P);
-  while (n > 1 && n * g.slice > SL_BUF) --n;
-  return n;
+  const int block = sl_block(g.P), most = SL_BUF / g.slice, n = block < most ? block : most;
+  return n < 1 ? 1 : n;
 }
 
 // buf <- m applied to the bond of dimension q and stride ks, in place, for ncol
