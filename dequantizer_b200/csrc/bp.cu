@@ -853,7 +853,7 @@ struct SweepItem {
 // cycles an SM) and a level has 16 to 194 of them.
 // One CTA per SM: 120 KB with the table, and 217 registers a thread (128, for a
 // second one that never fits, spilled).
-// Measured at bond 32 on the 127-qubit heavy-hex lattice (72 levels): 1,677 us, 1,838 us
+// Measured at bond 32 on the 127-qubit heavy-hex lattice (72 levels): 1,670 us, 1,838 us
 // with the spills; one slice an item and generic arithmetic 3,252 us, without the
 // table 2,107 us.
 __global__ void __launch_bounds__(SL_THREADS) bp_sweep_sliced_kernel(
