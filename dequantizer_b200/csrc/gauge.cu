@@ -157,8 +157,8 @@ __global__ void __launch_bounds__(GAUGE_THREADS) vidal_edges_kernel(dqz_graph_t 
 
 // One warp per edge (chi <= WARP_MAX_CHI), the factored form (edge_svd.cuh);
 // edges it does not cover get ES_MARK in lambda[0]. Measured at 1,536 edges of
-// bond 16 (random 3-regular graph, 1,024 nodes): 193 us, 1,572 us with the
-// eigendecompositions; at bond 3 41 and 68 us; at bond 2 21 and 20 us.
+// bond 16 (random 3-regular graph, 1,024 nodes): 182 us, 1,572 us with the
+// eigendecompositions; at bond 3 35 and 68 us; at bond 2 22 and 20 us.
 constexpr int ES_WARPS = 4;
 __global__ void __launch_bounds__(32 * ES_WARPS, 4) vidal_edges_factored_kernel(dqz_graph_t g,
                                                                                  const cd *__restrict__ n2e,
